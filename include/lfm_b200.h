@@ -152,6 +152,36 @@ int lfm_leapfrog_complex_f32(const float* psi_r, float* psi_r_prev_io, const flo
                              int N, double dt2, double kappa, double lambda_self,
                              double chi0, double e0_sq, double epsilon_w, void* stream);
 
+/* `steps` resident steps of a small REAL or COMPLEX lattice in one launch, the
+ * state held in the SMs' shared memory between them (the same bits as `steps`
+ * calls of lfm_leapfrog_real_f32 / _complex_f32).  Slot s of each field is
+ * f_s0 (current) and f_s1 (previous) before the call; after it the current
+ * fields are in the s0 slots if `steps` is even, in the s1 slots if odd, and
+ * the other slot holds the level before, undamped.  psi_i slots are null at
+ * REAL.  sync: lfm_leapfrog_run_words() 32-bit words of device memory (16-byte
+ * aligned), zeroed once by the caller and then used by one lattice's calls only,
+ * one at a time.
+ * Returns LFM_ERR_UNSUPPORTED (nothing launched) when the lattice does not fit
+ * on chip, steps < 2, a slot of an N % 4 == 0 lattice is not 16-byte aligned, or a
+ * step path or tile was forced with lfm_set_step_path / lfm_tune_set: the
+ * caller then takes the single steps. */
+int lfm_leapfrog_run_f32(int level, int steps, float* psi_r_s0, float* psi_r_s1,
+                         float* psi_i_s0, float* psi_i_s1, float* chi_s0, float* chi_s1,
+                         const float* mask_table, const lfm_mask_lut* lut, int damp_prev, int N,
+                         double dt2, double kappa, double lambda_self, double chi0, double e0_sq,
+                         double epsilon_w, unsigned int* sync, void* stream);
+
+/* Words of that workspace for an N^3 lattice on the current device; 0 if it does
+ * not fit on chip. */
+int lfm_leapfrog_run_words(int level, int N, long long* words);
+
+/* The cut of an N^3 lattice over `sms` SMs that lfm_leapfrog_run_f32 uses, for
+ * inspection and tests (no device needed): plan[0..7] = blocks along i, blocks
+ * along j, rows of the largest block along i and j, cells per thread, plane
+ * segments, threads, shared-memory bytes.  LFM_ERR_UNSUPPORTED if it does not
+ * fit. */
+int lfm_leapfrog_run_plan(int level, int N, int sms, int* plan);
+
 /* sa: raw (unclipped) S_a fields from lfm_helmholtz_sa_f32 of this step's
  * psi, or NULL when kappa_tube == 0; the kernel clips them at 0 on read. */
 int lfm_leapfrog_color_f32(const float* psi_r, float* psi_r_prev_io, const float* psi_i,

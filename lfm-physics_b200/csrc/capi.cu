@@ -19,6 +19,8 @@
 #include "lfm_batch.h"
 #include "lfm_kernels.h"
 #include "lfm_metrics.h"
+#include "lfm_resident.h"
+#include "lfm_tune.h"
 
 // Device status word: bounded device-side waits OR an LFM_ERR_* code into
 // it when they give up (read back with lfm_device_status).
@@ -636,6 +638,88 @@ int lfm_leapfrog_complex_f32(const float* psi_r, float* psi_r_prev_io, const flo
   a.lut = device_lut(mask_table, lut);
   a.damp_prev = damp_prev ? 1 : 0;
   return run_step(a, static_cast<cudaStream_t>(stream));
+}
+
+int lfm_leapfrog_run_words(int level, int N, long long* words) {
+  if (!words) return fail(LFM_ERR_INVALID_ARG, "null output");
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return cuda_fail(e, "device attributes");
+  lfm::ResidentPlan p;
+  *words = lfm::resident_plan(level, N, sms, &p) ? p.words : 0;
+  return LFM_OK;
+}
+
+int lfm_leapfrog_run_plan(int level, int N, int sms, int* plan) {
+  if (!plan) return fail(LFM_ERR_INVALID_ARG, "null output");
+  lfm::ResidentPlan p;
+  if (!lfm::resident_plan(level, N, sms, &p))
+    return fail(LFM_ERR_UNSUPPORTED, "N=%d level=%d does not fit on %d SMs", N, level, sms);
+  const int v[8] = {p.nbi, p.nbj, p.NI, p.NJ, p.V, p.segs, p.threads, p.smem};
+  std::copy(v, v + 8, plan);
+  return LFM_OK;
+}
+
+int lfm_leapfrog_run_f32(int level, int steps, float* psi_r_s0, float* psi_r_s1,
+                         float* psi_i_s0, float* psi_i_s1, float* chi_s0, float* chi_s1,
+                         const float* mask_table, const lfm_mask_lut* lut, int damp_prev, int N,
+                         double dt2, double kappa, double lambda_self, double chi0, double e0_sq,
+                         double epsilon_w, unsigned int* sync, void* stream) {
+  int rc = check_n(N);
+  if (rc) return rc;
+  const bool cx = level == LFM_COMPLEX;
+  if (level != LFM_REAL && !cx)
+    return fail(LFM_ERR_UNSUPPORTED, "run: level %d (REAL and COMPLEX only)", level);
+  if (!psi_r_s0 || !psi_r_s1 || !chi_s0 || !chi_s1 || !sync || (cx && (!psi_i_s0 || !psi_i_s1)))
+    return fail(LFM_ERR_INVALID_ARG, "null buffer");
+  rc = check_lut(mask_table, lut, N);
+  if (rc) return rc;
+  const size_t b = sizeof(float) * (size_t)N * N * N;
+  std::vector<Span> slots = {{psi_r_s0, b}, {psi_r_s1, b}, {chi_s0, b}, {chi_s1, b}};
+  if (cx) {
+    slots.push_back({psi_i_s0, b});
+    slots.push_back({psi_i_s1, b});
+  }
+  rc = check_disjoint({}, slots);
+  if (rc) return rc;
+  if (steps < 2) return fail(LFM_ERR_UNSUPPORTED, "run: %d steps", steps);
+  lfm::TileConfig forced;
+  if (g_path.load() != 0 || lfm::tune_lookup(level, N, &forced))
+    return fail(LFM_ERR_UNSUPPORTED, "run: a step path or tile is forced");
+  if (!aligned16(sync)) return fail(LFM_ERR_ALIGNMENT, "run: workspace alignment");
+  for (const Span& s : slots)
+    if (N % 4 == 0 && !aligned16(s.p)) return fail(LFM_ERR_UNSUPPORTED, "run: slot alignment");
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return cuda_fail(e, "device attributes");
+  lfm::ResidentArgs a{};
+  if (!lfm::resident_plan(level, N, sms, &a.plan))
+    return fail(LFM_ERR_UNSUPPORTED, "run: N=%d level=%d does not fit on chip", N, level);
+  rc = status_word(&a.status);
+  if (rc) return rc;
+  a.level = level;
+  a.N = N;
+  a.steps = steps;
+  a.damp_first = damp_prev ? 1 : 0;
+  a.c = lfm::make_step_consts(dt2, kappa, lambda_self, chi0, e0_sq, cx ? epsilon_w : 0.0, 0, 0,
+                              0, 0);
+  a.lut = device_lut(mask_table, lut);
+  a.sync = sync;
+  a.packets = reinterpret_cast<ulonglong2*>(sync + 4);
+  int f = 0;
+  auto field = [&](float* s0, float* s1) {
+    a.cur[f] = a.even[f] = s0;
+    a.prev[f] = a.odd[f] = s1;
+    ++f;
+  };
+  field(psi_r_s0, psi_r_s1);
+  if (cx) field(psi_i_s0, psi_i_s1);
+  field(chi_s0, chi_s1);
+  e = lfm::launch_resident(a, static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) return cuda_fail(e, "resident run launch");
+  return LFM_OK;
 }
 
 int lfm_poisson_chi_f32(lfm_context* ctx, int level, const float* psi_r, const float* psi_i,

@@ -1,0 +1,47 @@
+// Many steps of one lattice held on chip in one launch (resident.cu).
+#pragma once
+
+#include <cstdint>
+#include <cuda_runtime.h>
+
+#include "lfm_math.cuh"
+
+namespace lfm {
+
+// How a lattice is cut over the SMs: nbi x nbj blocks of whole k rows, block
+// (bi, bj) owning planes [bi N / nbi, (bi+1) N / nbi) and rows likewise; NI x
+// NJ the largest block.  A CTA's threads are `segs` plane segments x the rows
+// of a plane x ceil(N / V) groups of V cells.
+struct ResidentPlan {
+  int nbi = 0, nbj = 0, NI = 0, NJ = 0;
+  int V = 0, segs = 0, threads = 0;
+  int RS = 0;    // floats of a shared-memory row
+  int smem = 0;  // bytes of dynamic shared memory
+  long long words = 0;  // 32-bit words of the workspace: 4 counters, two exchange buffers
+};
+
+// The plan of an N^3 lattice at `level` on `sms` SMs; false if its state does
+// not fit on chip.
+bool resident_plan(int level, int N, int sms, ResidentPlan* plan);
+
+struct ResidentArgs {
+  int level, N;
+  int steps, damp_first;
+  ResidentPlan plan;
+  // Psi_r, (Psi_i,) chi at the current time level and the one before; time
+  // levels of even / odd distance from the current one are stored to even /
+  // odd (for the two-slot layout: even = cur, odd = prev).
+  const float* cur[3];
+  const float* prev[3];
+  float* even[3];
+  float* odd[3];
+  StepConsts c;
+  MaskLut lut;
+  uint32_t* sync;        // workspace words 0 (time base) and 1 (retired CTAs)
+  ulonglong2* packets;   // the two exchange buffers, from workspace word 4 on
+  int* status;
+};
+
+cudaError_t launch_resident(const ResidentArgs& a, cudaStream_t stream);
+
+}  // namespace lfm

@@ -32,6 +32,7 @@
 #include "lfm_cells.cuh"
 #include "lfm_batch.h"
 #include "lfm_kernels.h"
+#include "lfm_queue.cuh"
 #include "lfm_tune.h"
 
 namespace lfm {
@@ -43,7 +44,6 @@ constexpr int kMaxStencil = 7;
 constexpr int kPlain = 0, kComp = 1, kSplit = 2;
 constexpr int kMaxPoint = 11;
 constexpr int kMaxStages = 6;
-constexpr uint64_t kWaitLimitNs = 1000000000ull;  // 1 s per wait
 constexpr uint64_t kDrainLimitNs = 100000000ull;  // 0.1 s per stage when draining
 
 struct TmaParams {
@@ -126,12 +126,6 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-__device__ __forceinline__ uint64_t now_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
 // try_wait that may suspend the thread for up to hint_ns until the phase
 // completes (it resumes as soon as it does), so a waiting warp sleeps instead
 // of spinning on the issue slots of the warps that have their data.
@@ -162,38 +156,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     if (SLEEP ? mbar_try_wait_sleep(bar, parity, kSleepHintNs) : mbar_try_wait(bar, parity))
       return true;
     if (now_ns() - t0 > limit_ns) return false;
-  }
-}
-
-// ---- vector helpers ------------------------------------------------------------
-template <int V>
-struct Vec {
-  float v[V];
-};
-
-template <int V>
-__device__ __forceinline__ Vec<V> lds(const float* smem, int off) {
-  Vec<V> r;
-  if constexpr (V == 4) {
-    const float4 t = *reinterpret_cast<const float4*>(smem + off);
-    r.v[0] = t.x; r.v[1] = t.y; r.v[2] = t.z; r.v[3] = t.w;
-  } else if constexpr (V == 2) {
-    const float2 t = *reinterpret_cast<const float2*>(smem + off);
-    r.v[0] = t.x; r.v[1] = t.y;
-  } else {
-    r.v[0] = smem[off];
-  }
-  return r;
-}
-
-template <int V>
-__device__ __forceinline__ void stg(float* p, const float (&x)[V]) {
-  if constexpr (V == 4) {
-    *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
-  } else if constexpr (V == 2) {
-    *reinterpret_cast<float2*>(p) = make_float2(x[0], x[1]);
-  } else {
-    *p = x[0];
   }
 }
 
@@ -621,13 +583,6 @@ __global__ void __launch_bounds__(512) tma_step_kernel(const __grid_constant__ T
 // renaming).  Neighbours k0-1 and k0+V are plain scalar loads.  A stage is
 // dead once its plane has been the centre plane, so it is refilled one plane
 // earlier than in tma_step_kernel: S stages keep S-2 planes in flight.
-template <int V>
-struct QPlane {
-  Vec<V> m, z, p;        // rows j-1, j, j+1
-  float zl, zr;          // row j at k0-1, k0+V
-  float ml, mr, pl, pr;  // rows j-1, j+1 at k0-1, k0+V (loaded when centre)
-};
-
 struct QLane {
   int j, k0;                               // the thread's row and first cell
   int o_m, o_z, o_p;                       // row offsets at k0 in a field block
@@ -718,38 +673,6 @@ __device__ __forceinline__ void q_centre(QPlane<V>& q, const float* smem, int ba
   q.mr = smem[base + L.o_mr];
   q.pl = smem[base + L.o_pl];
   q.pr = smem[base + L.o_pr];
-}
-
-template <int V>
-__device__ __forceinline__ S19 q_s19(const QPlane<V>& M, const QPlane<V>& A, const QPlane<V>& P,
-                                     int e) {
-  S19 s;
-  s.c = A.z.v[e];
-  s.im = M.z.v[e];
-  s.ip = P.z.v[e];
-  s.jm = A.m.v[e];
-  s.jp = A.p.v[e];
-  s.km = e > 0 ? A.z.v[e - 1] : A.zl;
-  s.kp = e < V - 1 ? A.z.v[e + 1] : A.zr;
-  s.imjm = M.m.v[e];
-  s.imjp = M.p.v[e];
-  s.ipjm = P.m.v[e];
-  s.ipjp = P.p.v[e];
-  s.imkm = e > 0 ? M.z.v[e - 1] : M.zl;
-  s.imkp = e < V - 1 ? M.z.v[e + 1] : M.zr;
-  s.ipkm = e > 0 ? P.z.v[e - 1] : P.zl;
-  s.ipkp = e < V - 1 ? P.z.v[e + 1] : P.zr;
-  s.jmkm = e > 0 ? A.m.v[e - 1] : A.ml;
-  s.jmkp = e < V - 1 ? A.m.v[e + 1] : A.mr;
-  s.jpkm = e > 0 ? A.p.v[e - 1] : A.pl;
-  s.jpkp = e < V - 1 ? A.p.v[e + 1] : A.pr;
-  return s;
-}
-
-__device__ __forceinline__ Faces faces_of(const S19& s) {
-  Faces f;
-  f.im = s.im; f.ip = s.ip; f.jm = s.jm; f.jp = s.jp; f.km = s.km; f.kp = s.kp;
-  return f;
 }
 
 // Stencil and point fields of the march: Psi components and chi (split chi:

@@ -71,6 +71,10 @@ _SIGNATURES = {
     "lfm_context_destroy": [_P],
     "lfm_leapfrog_real_f32": [_P] * 5 + [POINTER(MaskLut), c_int, c_int] + [_D] * 5 + [_P],
     "lfm_leapfrog_complex_f32": [_P] * 7 + [POINTER(MaskLut), c_int, c_int] + [_D] * 6 + [_P],
+    "lfm_leapfrog_run_f32": [c_int, c_int] + [_P] * 7 + [POINTER(MaskLut), c_int, c_int]
+    + [_D] * 6 + [_P, _P],
+    "lfm_leapfrog_run_words": [c_int, c_int, POINTER(ctypes.c_longlong)],
+    "lfm_leapfrog_run_plan": [c_int, c_int, c_int, POINTER(c_int)],
     "lfm_leapfrog_color_f32": [_P] * 7 + [POINTER(MaskLut), c_int, c_int] + [_D] * 10
     + [_P, _P],
     "lfm_leapfrog_color_energy_f32": [_P] * 7 + [POINTER(MaskLut), c_int, c_int] + [_D] * 10
@@ -153,6 +157,26 @@ def call(name: str, *args) -> None:
 def set_step_path(path: int) -> None:
     """Choose the step kernel: 0 automatic, 1 direct, 2 fused 2.5D only."""
     call("lfm_set_step_path", int(path))
+
+
+def run_workspace(level: int, N: int, device):
+    """Zeroed workspace of lfm_leapfrog_run_f32 for one lattice; empty if it does not fit."""
+    import torch
+
+    n = ctypes.c_longlong(0)
+    with torch.cuda.device(device):
+        call("lfm_leapfrog_run_words", int(level), int(N), ctypes.byref(n))
+    return torch.zeros(n.value, dtype=torch.int32, device=device)
+
+
+def run_steps(*args) -> bool:
+    """lfm_leapfrog_run_f32: True if the steps were launched, False if the lattice
+    has to take single steps (LFM_ERR_UNSUPPORTED); raises on any other error."""
+    rc = load().lfm_leapfrog_run_f32(*args)
+    if rc == LFM_ERR_UNSUPPORTED:
+        return False
+    check(rc, "lfm_leapfrog_run_f32")
+    return True
 
 
 def tune_set(level: int, N: int, tj: int, stages: int, ic: int = 0, vec: int = 0) -> None:

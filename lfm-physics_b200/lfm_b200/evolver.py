@@ -86,6 +86,7 @@ class Evolver:
             self._absorb_psi = self._absorb
 
         self._energy_ok = False
+        self._run_sync = None  # workspace of the on-chip runs, made on first use
         if self._mode == "resident":
             self._table_dev = self._table.to_device(self.device)
             self._desc = self._table.desc
@@ -343,8 +344,42 @@ class Evolver:
             self._pair_graph()
         self._cur = saved
 
+    run_block = 4096
+    """Most steps per launch of a lattice that fits on chip (bounds a launch's length)."""
+
+    def _run_on_chip(self, steps: int) -> bool:
+        """`steps` steps with the state held on chip (lfm_leapfrog_run_f32); False if the
+        lattice does not fit, or a step path or tile is forced."""
+        if self._level == FieldLevel.COLOR:
+            return False
+        cfg = self.config
+        if self._run_sync is None:
+            self._run_sync = _lib.run_workspace(int(self._level), self.N, self.device)
+        if self._run_sync.numel() == 0:
+            return False
+        cur, prv = self._cur, 1 - self._cur
+        pi = ((self._pi[cur].data_ptr(), self._pi[prv].data_ptr()) if self._has_imag
+              else (None, None))
+        if not _lib.run_steps(
+                int(self._level), steps, self._pr[cur].data_ptr(), self._pr[prv].data_ptr(), *pi,
+                self._chi[cur].data_ptr(), self._chi[prv].data_ptr(), self._table_dev.data_ptr(),
+                ctypes.byref(self._desc), 1 if self._damp else 0, self.N, float(self._dt2),
+                float(cfg.kappa), float(cfg.lambda_self), float(cfg.chi0), float(cfg.e0_sq),
+                float(cfg.epsilon_w), self._run_sync.data_ptr(), _stream_handle(self.device)):
+            return False
+        if steps % 2:
+            self._cur = prv
+            self._use_buffer_A = not self._use_buffer_A
+        self._damp = True
+        self.step += steps
+        return True
+
     def _evolve_graphed(self, steps: int) -> None:
         self._dt2 = self.config.dt**2
+        while steps >= 2 and self._run_on_chip(min(steps, self.run_block)):
+            steps -= min(steps, self.run_block)
+        if steps < 1:
+            return
         done = 0
         if not self._damp or (self._sa_on and not self._energy_ok):
             # first step after a host write: the kernel must not damp prev, and
