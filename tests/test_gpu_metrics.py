@@ -111,3 +111,55 @@ def test_metrics_reject_bad_arguments(be):
         device_metrics(be.context.handle, 1, 8, chi, None, None, None, chi, 0.02)
     with pytest.raises(LfmError):
         device_metrics(be.context.handle, 0, 8, chi, None, None, None, chi, -1.0)
+
+
+@pytest.mark.parametrize("level", [0, 1, 2])
+@pytest.mark.parametrize("N,shift,with_prev", [(4, 0, True), (9, 0, True), (30, 0, False),
+                                               (32, 0, True), (36, 1, True), (68, 0, True),
+                                               (132, 0, True), (65, 0, True)])
+def test_metrics_at_the_edges_of_the_march(be, level, N, shift, with_prev):
+    """Four cells a thread (N % 4 == 0, 16-byte aligned) and one (odd edges, shifted
+    fields), around the plane counts of a march, against numpy in float64.  Sums of n
+    terms in another order differ by at most about sqrt(n) 2^-53 relative: 1e-12 holds."""
+    import torch
+
+    from lfm_b200.metrics import device_metrics
+
+    rng = np.random.default_rng(N + level)
+    colours = 3 if level == 2 else 1
+    shape = (colours, N, N, N)
+
+    def dev(a):
+        flat = torch.zeros(a.size + shift, dtype=torch.float32, device=be.device)
+        flat[shift:] = torch.from_numpy(a.ravel()).to(be.device)
+        return flat[shift:]
+
+    f = lambda: rng.standard_normal(shape).astype(np.float32)  # noqa: E731
+    parts = [f() for _ in range(1 if level == 0 else 2)]
+    prevs = [f() for _ in parts] if with_prev else [None for _ in parts]
+    chi = (18.0 + rng.standard_normal((N, N, N))).astype(np.float32)
+    d = [dev(p) for p in parts] + [None]
+    dp = [None if p is None else dev(p) for p in prevs] + [None]
+    m = device_metrics(be.context.handle, level, N, d[0], dp[0], d[1], dp[1], dev(chi), 0.02, 1.0,
+                       0.3)
+    c64 = chi.astype(np.float64)
+    kin = grad = psi2 = 0.0
+    for p, q in zip(parts, prevs):
+        for a in range(colours):
+            v = p[a].astype(np.float64)
+            psi2 = psi2 + v * v
+            grad += 0.5 * sum(float((g * g).sum()) for g in np.gradient(v))
+            if q is not None:
+                kin += 0.5 * float((((v - q[a].astype(np.float64)) / 0.02) ** 2).sum())
+    x = np.arange(N) - N / 2.0
+    dist = np.sqrt(x[:, None, None] ** 2 + x[None, :, None] ** 2 + x[None, None, :] ** 2)
+    inner = c64[dist <= N / 2.0 * 0.7]
+    want = {"energy_kinetic": kin, "energy_gradient": grad,
+            "energy_potential": 0.5 * float((c64 * c64 * psi2).sum()),
+            "psi_sq_total": float(psi2.sum()), "chi_mean": inner.mean(), "chi_std": inner.std()}
+    for k, v in want.items():
+        assert m[k] == pytest.approx(v, rel=1e-12), k
+    assert m["chi_min"] == inner.min() and m["chi_max"] == inner.max()
+    assert m["interior_cells"] == inner.size and m["nonfinite_cells"] == 0
+    assert m["well_fraction"] == (inner < 17.0).mean()
+    assert m["void_fraction"] == (inner > 18.0).mean()
