@@ -114,31 +114,55 @@ struct Block {
 template <int LEVEL>
 constexpr int kFieldFloats = LEVEL == LFM_REAL ? 22656 : 16448;
 
-struct RowOff {
-  int m, z, p;  // rows jr-1, jr, jr+1 of a plane, at the thread's first cell
-};
-
 // A thread's cells: k0 .. k0+V-1 of row jr, planes [pa, pb).
 struct Cells {
   int jr, kg, groups, k0;
   int pa, pb;
-  bool whole;  // all V cells lie in the row
+  bool first, last;  // the row's first / last group: its end copies are this thread's
+  bool edge_row;     // row 0 or nj-1 of the block
 };
 
-__device__ __forceinline__ RowOff rows_of(const Block& B, int cur, int ii, const Cells& T) {
-  RowOff o;
-  const int own = 4 + T.k0 + cur * B.SLOT + (ii * B.NJ + T.jr) * B.RS;
-  const int side = 4 + T.k0 + 2 * B.SLOT + (2 * B.NJ2 + 2 * ii) * B.RS;
-  const int end = 4 + T.k0 + 2 * B.SLOT + ((ii < 0 ? 0 : B.NJ2) + T.jr) * B.RS;
-  const bool halo = ii < 0 || ii >= B.ni;
-  o.z = halo ? end + B.RS : own;
-  o.m = halo ? end : (T.jr > 0 ? own - B.RS : side);
-  o.p = halo ? end + 2 * B.RS : (T.jr < B.nj - 1 ? own + B.RS : side + B.RS);
+// Offsets of the thread's first cell in rows jr-1, jr, jr+1 of a plane.
+struct RowOff {
+  int m, z, p;
+};
+
+// Walks a thread's rows plane by plane: own planes lie NJ rows apart, the halo rows
+// beside them (under m at row 0, under p at row nj-1) two rows apart, and the planes
+// before and after the block among the halo rows.
+struct RowWalk {
+  RowOff next;     // of the next own plane
+  int dz, dm, dp;  // to the plane after
+};
+
+__device__ __forceinline__ RowWalk walk_from(const Block& B, const Cells& T, int cur, int ii) {
+  RowWalk w;
+  const int halo = 4 + T.k0 + 2 * B.SLOT, side = halo + (2 * B.NJ2 + 2 * ii) * B.RS;
+  w.dz = B.NJ * B.RS;
+  w.dm = T.jr > 0 ? w.dz : 2 * B.RS;
+  w.dp = T.jr < B.nj - 1 ? w.dz : 2 * B.RS;
+  w.next.z = 4 + T.k0 + cur * B.SLOT + (ii * B.NJ + T.jr) * B.RS;
+  w.next.m = T.jr > 0 ? w.next.z - B.RS : side;
+  w.next.p = T.jr < B.nj - 1 ? w.next.z + B.RS : side + B.RS;
+  return w;
+}
+
+__device__ __forceinline__ RowOff halo_plane(const Block& B, const Cells& T, bool after) {
+  const int m = 4 + T.k0 + 2 * B.SLOT + ((after ? B.NJ2 : 0) + T.jr) * B.RS;
+  return RowOff{m, m + B.RS, m + 2 * B.RS};
+}
+
+__device__ __forceinline__ RowOff step_rows(RowWalk& w) {
+  const RowOff o = w.next;
+  w.next.m += w.dm;
+  w.next.z += w.dz;
+  w.next.p += w.dp;
   return o;
 }
 
 struct Step {
   int cur;         // shared-memory slot of the current time level
+  int to_prev;     // from a cell of the current slot to the other one's
   bool damp;       // previous Psi is stored undamped
   bool store;      // one of the last two time levels: to the field slots
   uint32_t t;      // the new time level
@@ -170,53 +194,46 @@ __device__ __forceinline__ void load_sides(QPlane<V>& q, const float* f, const R
   q.pr = f[o.p + V];
 }
 
-// Stores a thread's V values at its place `p` of a row of N cells in global memory.
-template <int V>
-__device__ __forceinline__ void store_global(float* p, const float (&x)[V], int N, int k0) {
-  if ((N & (V - 1)) == 0) {
-    stg<V>(p, x);
+// Stores a thread's two values at its place `p` of a row in global memory.  EVEN: N
+// is even, so the row's last group has both cells and rows start on 8 bytes.
+template <bool EVEN>
+__device__ __forceinline__ void store_global(float* p, const float (&x)[2], const Cells& T) {
+  if constexpr (EVEN) {
+    stg<2>(p, x);
   } else {
-#pragma unroll
-    for (int e = 0; e < V; ++e)
-      if (k0 + e < N) p[e] = x[e];
+    p[0] = x[0];
+    if (!T.last) p[1] = x[1];
   }
 }
 
 // The same in shared memory, with the copies beyond the row's ends.
-template <int V>
-__device__ __forceinline__ void store_row(float* p, const float (&x)[V], const Block& B,
+template <bool EVEN>
+__device__ __forceinline__ void store_row(float* p, const float (&x)[2], const Block& B,
                                           const Cells& T) {
-  if (T.whole) {
-    stg<V>(p, x);
-  } else {
-#pragma unroll
-    for (int e = 0; e < V; ++e)
-      if (T.k0 + e < B.N) p[e] = x[e];
-  }
-  if (T.k0 == 0) p[B.N] = x[0];
-  if (T.k0 + V >= B.N) {
-    float last = x[V - 1];
-#pragma unroll
-    for (int e = 0; e < V - 1; ++e)
-      if (T.k0 + e == B.N - 1) last = x[e];
-    p[-T.k0 - 1] = last;
-  }
+  if (EVEN || !T.last)
+    stg<2>(p, x);
+  else
+    p[0] = x[0];
+  if (T.first) p[B.N] = x[0];
+  if (T.last) p[-T.k0 - 1] = EVEN ? x[1] : x[0];
 }
 
-template <int LEVEL, int V, int PA, int PB, int PC>
+template <int LEVEL, bool EVEN, int PA, int PB, int PC>
 __device__ __forceinline__ void plane(const StepConsts& c, float* sm, const Block& B,
                                       const Cells& T, const Step& S,
-                                      QPlane<V> (&Q)[kFields<LEVEL>][3], int ii, RowOff& centre) {
-  constexpr int NS = kFields<LEVEL>;
-  constexpr int FS = kFieldFloats<LEVEL>;
-  const RowOff nxt = rows_of(B, S.cur, ii + 1, T);
+                                      QPlane<kCells> (&Q)[kFields<LEVEL>][3], int ii,
+                                      RowOff& centre, RowWalk& walk, int& mask_at) {
+  constexpr int NS = kFields<LEVEL>, FS = kFieldFloats<LEVEL>, V = kCells;
+  const RowOff nxt = ii + 1 < B.ni ? walk.next : halo_plane(B, T, true);
+  step_rows(walk);
 #pragma unroll
   for (int f = 0; f < NS; ++f) {
     load_rows<V>(Q[f][PC], sm + f * FS, nxt);
     load_sides<V>(Q[f][PB], sm + f * FS, centre);
   }
-  const int prv = centre.z + (1 - 2 * S.cur) * B.SLOT;
-  const Vec<V> mask = lds<V>(sm + NS * FS, (ii * B.NJ + T.jr) * B.N4 + T.k0);
+  const int prv = centre.z + S.to_prev;
+  const Vec<V> mask = lds<V>(sm + NS * FS, mask_at);
+  mask_at += B.NJ * B.N4;
   Vec<V> old[NS];
 #pragma unroll
   for (int f = 0; f < NS; ++f) old[f] = lds<V>(sm + f * FS, prv);
@@ -252,8 +269,8 @@ __device__ __forceinline__ void plane(const StepConsts& c, float* sm, const Bloc
     }
   }
 #pragma unroll
-  for (int f = 0; f < NS; ++f) store_row<V>(sm + f * FS + prv, out[f], B, T);
-  if (ii == 0 || ii == B.ni - 1 || T.jr == 0 || T.jr == B.nj - 1) {
+  for (int f = 0; f < NS; ++f) store_row<EVEN>(sm + f * FS + prv, out[f], B, T);
+  if (T.edge_row || ii == 0 || ii == B.ni - 1) {
     constexpr int NP = kPackets<LEVEL, V>;
     ulonglong2* d = S.out + outer_row(ii, T.jr, B.ni, B.nj, B.NI, B.NJ) * NP * T.groups + T.kg;
 #pragma unroll
@@ -271,7 +288,7 @@ __device__ __forceinline__ void plane(const StepConsts& c, float* sm, const Bloc
   if (S.store) {
     const int g = ((B.i0 + ii) * B.N + B.j0 + T.jr) * B.N + T.k0;
 #pragma unroll
-    for (int f = 0; f < NS; ++f) store_global<V>(S.dst[f] + g, out[f], B.N, T.k0);
+    for (int f = 0; f < NS; ++f) store_global<EVEN>(S.dst[f] + g, out[f], T);
   }
   centre = nxt;
 }
@@ -280,11 +297,11 @@ __device__ __forceinline__ void plane(const StepConsts& c, float* sm, const Bloc
 // A thread takes the V cells of group kg of every rows_a_round-th row, the first
 // kBatch rows at once: their packets are polled before the CTA's barrier, behind
 // which every thread is done with the halo of the time before.
-template <int LEVEL, int V>
+template <int LEVEL, bool EVEN>
 __device__ __forceinline__ bool receive(float* sm, const Block& B, const Cells& T,
                                         const ulonglong2* in, const int* halo_src, int HR,
                                         uint32_t t, int first, int rows_a_round) {
-  constexpr int NS = kFields<LEVEL>, NP = kPackets<LEVEL, V>, kBatch = 4;
+  constexpr int V = kCells, NS = kFields<LEVEL>, NP = kPackets<LEVEL, V>, kBatch = 4;
   constexpr int FS = kFieldFloats<LEVEL>;
   constexpr int LAST = NS * V - 3 * (NP - 1);  // values in a group's last packet
   bool ok = true, met = false;
@@ -338,7 +355,7 @@ __device__ __forceinline__ bool receive(float* sm, const Block& B, const Cells& 
         float v[V];
 #pragma unroll
         for (int e = 0; e < V; ++e) v[e] = x[u][(f * V + e) / 3].v[(f * V + e) % 3];
-        store_row<V>(row + f * FS, v, B, T);
+        store_row<EVEN>(row + f * FS, v, B, T);
       }
     }
   }
@@ -363,10 +380,10 @@ __device__ __forceinline__ void copy_rows(const float* src, float* dst, const in
   }
 }
 
-template <int LEVEL, int V, int THREADS>
+template <int LEVEL, bool EVEN, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1)
     resident_kernel(const __grid_constant__ ResidentArgs A) {
-  constexpr int NS = kFields<LEVEL>;
+  constexpr int V = kCells, NS = kFields<LEVEL>;
   extern __shared__ __align__(16) float sm[];
   __shared__ int s_abort;
   const ResidentPlan& L = A.plan;
@@ -451,7 +468,9 @@ __global__ void __launch_bounds__(THREADS, 1)
   const bool active = seg < L.segs;
   T.jr = (tid - seg * per_seg) / groups;
   T.k0 = T.kg * V;  // per_seg is a multiple of groups
-  T.whole = T.k0 + V <= A.N;
+  T.first = T.kg == 0;
+  T.last = T.kg == groups - 1;
+  T.edge_row = T.jr == 0 || T.jr == B.nj - 1;
   T.pa = active ? seg * B.ni / L.segs : 0;
   T.pb = active ? (seg + 1) * B.ni / L.segs : 0;
   const int rows_a_round = blockDim.x / groups;
@@ -463,6 +482,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   for (int s = 0; s < A.steps; ++s) {
     Step S;
     S.cur = s & 1;
+    S.to_prev = (1 - 2 * S.cur) * B.SLOT;
     S.damp = s > 0 || A.damp_first;
     S.store = s >= A.steps - 2;
     S.t = base + (uint32_t)(s + 1);
@@ -472,24 +492,25 @@ __global__ void __launch_bounds__(THREADS, 1)
     for (int f = 0; f < NS; ++f) S.dst[f] = (s & 1) ? A.even[f] : A.odd[f];
     if (T.pa < T.pb) {
       QPlane<V> Q[NS][3];
-      RowOff centre = rows_of(B, S.cur, T.pa - 1, T);
+      RowWalk walk = walk_from(B, T, S.cur, T.pa > 0 ? T.pa - 1 : 0);
+      RowOff centre = T.pa > 0 ? step_rows(walk) : halo_plane(B, T, false);
 #pragma unroll
       for (int f = 0; f < NS; ++f) load_rows<V>(Q[f][0], sm + f * FS, centre);
-      centre = rows_of(B, S.cur, T.pa, T);
+      centre = step_rows(walk);
 #pragma unroll
       for (int f = 0; f < NS; ++f) load_rows<V>(Q[f][1], sm + f * FS, centre);
-      int ii = T.pa;
+      int ii = T.pa, mask_at = (T.pa * B.NJ + T.jr) * B.N4 + T.k0;
       while (true) {
-        plane<LEVEL, V, 0, 1, 2>(A.c, sm, B, T, S, Q, ii, centre);
+        plane<LEVEL, EVEN, 0, 1, 2>(A.c, sm, B, T, S, Q, ii, centre, walk, mask_at);
         if (++ii >= T.pb) break;
-        plane<LEVEL, V, 1, 2, 0>(A.c, sm, B, T, S, Q, ii, centre);
+        plane<LEVEL, EVEN, 1, 2, 0>(A.c, sm, B, T, S, Q, ii, centre, walk, mask_at);
         if (++ii >= T.pb) break;
-        plane<LEVEL, V, 2, 0, 1>(A.c, sm, B, T, S, Q, ii, centre);
+        plane<LEVEL, EVEN, 2, 0, 1>(A.c, sm, B, T, S, Q, ii, centre, walk, mask_at);
         if (++ii >= T.pb) break;
       }
     }
     if (s + 1 == A.steps) break;
-    if (!receive<LEVEL, V>(sm, B, T, packets, halo_src, HR, S.t, first_row, rows_a_round)) {
+    if (!receive<LEVEL, EVEN>(sm, B, T, packets, halo_src, HR, S.t, first_row, rows_a_round)) {
       s_abort = 1;
       atomicOr(A.status, LFM_ERR_DEVICE_TIMEOUT);
     }
@@ -506,11 +527,11 @@ __global__ void __launch_bounds__(THREADS, 1)
   }
 }
 
-template <int LEVEL, int V, int THREADS>
+template <int LEVEL, bool EVEN, int THREADS>
 cudaError_t launch(const ResidentArgs& a, cudaStream_t stream) {
   static std::mutex mu;
   static int granted = 0;
-  const auto kernel = resident_kernel<LEVEL, V, THREADS>;
+  const auto kernel = resident_kernel<LEVEL, EVEN, THREADS>;
   {
     std::lock_guard<std::mutex> lk(mu);
     if (a.plan.smem > granted) {
@@ -525,10 +546,12 @@ cudaError_t launch(const ResidentArgs& a, cudaStream_t stream) {
                                      dim3(a.plan.threads), args, (size_t)a.plan.smem, stream);
 }
 
-template <int LEVEL, int V>
-cudaError_t launch_threads(const ResidentArgs& a, cudaStream_t stream) {
-  return a.plan.threads <= 384 ? launch<LEVEL, V, 384>(a, stream)
-                               : launch<LEVEL, V, 512>(a, stream);
+template <int LEVEL>
+cudaError_t launch_level(const ResidentArgs& a, cudaStream_t stream) {
+  const bool small = a.plan.threads <= 384, even = a.N % 2 == 0;
+  if (even)
+    return small ? launch<LEVEL, true, 384>(a, stream) : launch<LEVEL, true, 512>(a, stream);
+  return small ? launch<LEVEL, false, 384>(a, stream) : launch<LEVEL, false, 512>(a, stream);
 }
 
 }  // namespace
@@ -588,9 +611,8 @@ bool resident_plan(int level, int N, int sms, ResidentPlan* out) {
 }
 
 cudaError_t launch_resident(const ResidentArgs& a, cudaStream_t stream) {
-  if (a.level == LFM_REAL)
-    return launch_threads<LFM_REAL, kCells>(a, stream);
-  return launch_threads<LFM_COMPLEX, kCells>(a, stream);
+  return a.level == LFM_REAL ? launch_level<LFM_REAL>(a, stream)
+                             : launch_level<LFM_COMPLEX>(a, stream);
 }
 
 }  // namespace lfm
