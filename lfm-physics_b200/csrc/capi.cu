@@ -125,6 +125,11 @@ int run_step(lfm::StepArgs& a, cudaStream_t stream) {
       return fail(LFM_ERR_UNSUPPORTED, "no fused-kernel configuration for N=%d level=%d", a.N,
                   a.level);
   }
+  if (e == cudaErrorNotSupported && path == 0) {
+    // measured against the direct kernel at every size it takes (step_march.cu)
+    e = lfm::launch_march_step(a, stream);
+    if (e != cudaSuccess && e != cudaErrorNotSupported) return cuda_fail(e, "march step launch");
+  }
   if (e == cudaErrorNotSupported) {
     e = lfm::launch_direct_step(a, stream);
     if (e != cudaSuccess) return cuda_fail(e, "direct step launch");

@@ -52,6 +52,10 @@ struct StepArgs {
 
 cudaError_t launch_direct_step(const StepArgs& a, cudaStream_t stream);
 
+// Marching kernel through L1 for REAL and COMPLEX lattices of any N and alignment
+// (step_march.cu); cudaErrorNotSupported at COLOR.
+cudaError_t launch_march_step(const StepArgs& a, cudaStream_t stream);
+
 // Fused 2.5D kernel (N % 4 == 0).  Returns cudaErrorNotSupported when the
 // size has no tile configuration, so the caller can take the direct path.
 cudaError_t launch_tma_step(const StepArgs& a, cudaStream_t stream);
