@@ -290,11 +290,15 @@ template <int LEVEL, int MODE>
 cudaError_t launch(const StepArgs& a, bool pairs, cudaStream_t stream) {
   const int threads = kThreads<LEVEL>, range = a.slab ? a.i_hi - a.i_lo : a.N;
   const int tiles = (a.N * ((a.N + 1) / V) + threads - 1) / threads;
-  // Planes a march: long enough to amortise its two extra planes, with four CTAs or
-  // more a resident slot (2 x 148) so that the last wave is short.  Within 5 % of the
-  // best of 4, 8, 16, 24 and 32 planes at the sizes above but REAL 250^3 (8 %).
-  int planes = std::max(1, std::min(range, (int)((int64_t)tiles * range / (4 * 296))));
-  planes = std::min(std::max(planes, std::min(range, 4)), 32);
+  // Planes a march.  A small lattice takes as few as keep all CTAs resident (2 x 148;
+  // REAL 46^3: 4.2 us with 1 plane, 6.3 with 4).  Beyond four planes that way, long
+  // marches amortise their two extra planes, with four CTAs or more a resident slot
+  // so that the last wave is short: within 5 % of the best of 4, 8, 16, 24 and 32
+  // planes at the sizes above but REAL 250^3 (8 %).
+  const int64_t work = (int64_t)tiles * range;
+  int planes = (int)((work + 295) / 296);
+  if (planes > 4) planes = (int)std::min<int64_t>(32, std::max<int64_t>(4, work / (4 * 296)));
+  planes = std::min(planes, range);
   const unsigned grid = (unsigned)tiles * (unsigned)((range + planes - 1) / planes);
   if (pairs)
     march_step_kernel<LEVEL, MODE, true><<<grid, threads, 0, stream>>>(a, planes, tiles);
@@ -307,6 +311,9 @@ cudaError_t launch(const StepArgs& a, bool pairs, cudaStream_t stream) {
 
 cudaError_t launch_march_step(const StepArgs& a, cudaStream_t stream) {
   if (a.level != LFM_REAL && a.level != LFM_COMPLEX) return cudaErrorNotSupported;
+  // Below 32^3 the direct kernel's one-cell threads are done sooner (REAL 30^3: 3.2
+  // against 4.2 us a step; COMPLEX 15^3 to 30^3 4.2 either way).
+  if (a.N < 32) return cudaErrorNotSupported;
   // two cells a thread where every row starts on 8 bytes
   bool pairs = a.N % 2 == 0;
   const void* ptrs[] = {a.pr, a.pi, a.chi, a.pr_prev, a.pi_prev, a.chi_prev, a.pr_out, a.pi_out,
