@@ -160,7 +160,10 @@ int lfm_leapfrog_complex_f32(const float* psi_r, float* psi_r_prev_io, const flo
  * the other slot holds the level before, undamped.  psi_i slots are null at
  * REAL.  sync: lfm_leapfrog_run_words() 32-bit words of device memory (16-byte
  * aligned), zeroed once by the caller and then used by one lattice's calls only,
- * one at a time.
+ * one at a time.  stores: null, or in device memory, for every step s, the
+ * addresses stores[s * fields + f] of 16-byte aligned fields (psi_r, psi_i at
+ * COMPLEX, chi; apart from the slots) that the time level made by step s is stored
+ * to as well; null entries are skipped (all of a step's or none).
  * Returns LFM_ERR_UNSUPPORTED (nothing launched) when the lattice does not fit
  * on chip, steps < 2, a slot of an N % 4 == 0 lattice is not 16-byte aligned, or a
  * step path or tile was forced with lfm_set_step_path / lfm_tune_set: the
@@ -169,7 +172,17 @@ int lfm_leapfrog_run_f32(int level, int steps, float* psi_r_s0, float* psi_r_s1,
                          float* psi_i_s0, float* psi_i_s1, float* chi_s0, float* chi_s1,
                          const float* mask_table, const lfm_mask_lut* lut, int damp_prev, int N,
                          double dt2, double kappa, double lambda_self, double chi0, double e0_sq,
-                         double epsilon_w, unsigned int* sync, void* stream);
+                         double epsilon_w, float* const* stores, unsigned int* sync,
+                         void* stream);
+
+/* The same run out of place: the fields at the current and previous time level are
+ * only read, and the levels go to `stores` (not null) alone. */
+int lfm_advance_run_f32(int level, int steps, const float* psi_r, const float* psi_r_prev,
+                        const float* psi_i, const float* psi_i_prev, const float* chi,
+                        const float* chi_prev, float* const* stores, const float* mask_table,
+                        const lfm_mask_lut* lut, int damp_prev, int N, double dt2, double kappa,
+                        double lambda_self, double chi0, double e0_sq, double epsilon_w,
+                        unsigned int* sync, void* stream);
 
 /* Words of that workspace for an N^3 lattice on the current device; 0 if it does
  * not fit on chip. */

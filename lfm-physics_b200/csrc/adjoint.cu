@@ -66,11 +66,6 @@ struct TileSmem {
   float f[NF][HALO];  // ur, gx [, ui, pr, pi, wpr, wpi]
 };
 
-__device__ __forceinline__ int wrapmod(int x, int N) {
-  x %= N;
-  return x < 0 ? x + N : x;
-}
-
 template <int LEVEL>
 __global__ void __launch_bounds__(kThreads) adjoint_tile_kernel(const AdjArgs A) {
   extern __shared__ __align__(16) float sm_raw[];
@@ -84,13 +79,13 @@ __global__ void __launch_bounds__(kThreads) adjoint_tile_kernel(const AdjArgs A)
   const int i0 = (t / tiles_j) * TI;
   const float c_w = -0.5f * A.eps_w * A.K * A.dt2;  // w(y) = c_w X(y) gXn(y)
 
-  // phase 1: point terms of the block and its halo
-  for (int h = threadIdx.x; h < HALO; h += kThreads) {
-    const int hk = h % HK, hj = (h / HK) % HJ, hi = h / (HK * HJ);
-    const int gi = wrapmod(i0 + hi - 1, N), gj = wrapmod(j0 + hj - 1, N),
-              gk = wrapmod(k0 + hk - 1, N);
-    const int64_t y = ((int64_t)gi * N + gj) * N + gk;
-    const float m = mask_from_q_flat(A.lut, qterm(gi, N) + qterm(gj, N) + qterm(gk, N));
+  // phase 1: point terms of the block and its halo.  A warp takes a row of 32 cells at
+  // a time (its i and j once for the warp), then the threads take the two cells beyond
+  // each row.
+  const auto wrap = [&](int x) { return x < 0 ? x + N : (x >= N ? x - N : x); };
+  const auto point = [&](int h, int qij, int64_t row, int gk) {
+    const int64_t y = row + gk;
+    const float m = mask_from_q_flat(A.lut, qij + qterm(gk, N));
     const float a = fsub(1.0f, m);
     // the clamp value the forward writes: mask*chi0 + a*(-chi0)
     const float clamped = fadd(fmul(m, A.chi0), fmul(a, A.neg_chi0));
@@ -106,6 +101,21 @@ __global__ void __launch_bounds__(kThreads) adjoint_tile_kernel(const AdjArgs A)
       S.f[5][h] = w * pr;
       S.f[6][h] = w * pi;
     }
+  };
+  // rows and columns past the lattice's end stand for the cells they wrap to: only the
+  // first of them is read, so one fold is enough (any further ones stay in range)
+  const int lane = threadIdx.x & 31;
+  const int gl = min(wrap(k0 + lane), N - 1);
+#pragma unroll 2
+  for (int r = threadIdx.x >> 5; r < HI * HJ; r += kThreads / 32) {
+    const int gi = min(wrap(i0 + r / HJ - 1), N - 1), gj = min(wrap(j0 + r % HJ - 1), N - 1);
+    point(r * HK + 1 + lane, qterm(gi, N) + qterm(gj, N), ((int64_t)gi * N + gj) * N, gl);
+  }
+  if (threadIdx.x < 2 * HI * HJ) {
+    const int r = threadIdx.x >> 1, side = threadIdx.x & 1;
+    const int gi = min(wrap(i0 + r / HJ - 1), N - 1), gj = min(wrap(j0 + r % HJ - 1), N - 1);
+    point(r * HK + side * (HK - 1), qterm(gi, N) + qterm(gj, N), ((int64_t)gi * N + gj) * N,
+          min(wrap(side ? k0 + TK : k0 - 1), N - 1));
   }
   __syncthreads();
 

@@ -666,40 +666,51 @@ int lfm_leapfrog_run_plan(int level, int N, int sms, int* plan) {
   return LFM_OK;
 }
 
-int lfm_leapfrog_run_f32(int level, int steps, float* psi_r_s0, float* psi_r_s1,
-                         float* psi_i_s0, float* psi_i_s1, float* chi_s0, float* chi_s1,
-                         const float* mask_table, const lfm_mask_lut* lut, int damp_prev, int N,
-                         double dt2, double kappa, double lambda_self, double chi0, double e0_sq,
-                         double epsilon_w, unsigned int* sync, void* stream) {
+}  // extern "C"
+
+namespace {
+
+// Checks and launches an on-chip run.  cur / prev: (psi_r, psi_i, chi) at the current
+// and previous time level; even / odd: where the last two time levels go, or null.
+int run_on_chip(int level, int steps, const float* const cur[3], const float* const prev[3],
+                float* const even[3], float* const odd[3], float* const* stores,
+                const float* mask_table, const lfm_mask_lut* lut, int damp_prev, int N, double dt2,
+                double kappa, double lambda_self, double chi0, double e0_sq, double epsilon_w,
+                unsigned int* sync, void* stream) {
   int rc = check_n(N);
   if (rc) return rc;
   const bool cx = level == LFM_COMPLEX;
   if (level != LFM_REAL && !cx)
     return fail(LFM_ERR_UNSUPPORTED, "run: level %d (REAL and COMPLEX only)", level);
-  if (!psi_r_s0 || !psi_r_s1 || !chi_s0 || !chi_s1 || !sync || (cx && (!psi_i_s0 || !psi_i_s1)))
-    return fail(LFM_ERR_INVALID_ARG, "null buffer");
+  if (!sync) return fail(LFM_ERR_INVALID_ARG, "null buffer");
+  if (!aligned16(sync)) return fail(LFM_ERR_ALIGNMENT, "run: workspace alignment");
   rc = check_lut(mask_table, lut, N);
   if (rc) return rc;
-  const size_t b = sizeof(float) * (size_t)N * N * N;
-  std::vector<Span> slots = {{psi_r_s0, b}, {psi_r_s1, b}, {chi_s0, b}, {chi_s1, b}};
-  if (cx) {
-    slots.push_back({psi_i_s0, b});
-    slots.push_back({psi_i_s1, b});
-  }
-  rc = check_disjoint({}, slots);
-  if (rc) return rc;
   if (steps < 2) return fail(LFM_ERR_UNSUPPORTED, "run: %d steps", steps);
+  lfm::ResidentArgs a{};
+  int nf = 0;
+  for (int f = 0; f < 3; ++f) {
+    if (f == 1 && !cx) continue;
+    if (!cur[f] || !prev[f]) return fail(LFM_ERR_INVALID_ARG, "null buffer");
+    a.cur[nf] = cur[f];
+    a.prev[nf] = prev[f];
+    a.even[nf] = even ? even[f] : nullptr;
+    a.odd[nf] = odd ? odd[f] : nullptr;
+    for (const float* p : {a.cur[nf], a.prev[nf], (const float*)a.even[nf], (const float*)a.odd[nf]})
+      if (N % 4 == 0 && !aligned16(p)) return fail(LFM_ERR_UNSUPPORTED, "run: slot alignment");
+    if (N % 2 == 0)
+      for (const float* p : {(const float*)a.even[nf], (const float*)a.odd[nf]})
+        if (reinterpret_cast<uintptr_t>(p) & 7u)
+          return fail(LFM_ERR_UNSUPPORTED, "run: slot alignment");
+    ++nf;
+  }
   lfm::TileConfig forced;
   if (g_path.load() != 0 || lfm::tune_lookup(level, N, &forced))
     return fail(LFM_ERR_UNSUPPORTED, "run: a step path or tile is forced");
-  if (!aligned16(sync)) return fail(LFM_ERR_ALIGNMENT, "run: workspace alignment");
-  for (const Span& s : slots)
-    if (N % 4 == 0 && !aligned16(s.p)) return fail(LFM_ERR_UNSUPPORTED, "run: slot alignment");
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return cuda_fail(e, "device attributes");
-  lfm::ResidentArgs a{};
   if (!lfm::resident_plan(level, N, sms, &a.plan))
     return fail(LFM_ERR_UNSUPPORTED, "run: N=%d level=%d does not fit on chip", N, level);
   rc = status_word(&a.status);
@@ -708,23 +719,55 @@ int lfm_leapfrog_run_f32(int level, int steps, float* psi_r_s0, float* psi_r_s1,
   a.N = N;
   a.steps = steps;
   a.damp_first = damp_prev ? 1 : 0;
+  a.stores = stores;
   a.c = lfm::make_step_consts(dt2, kappa, lambda_self, chi0, e0_sq, cx ? epsilon_w : 0.0, 0, 0,
                               0, 0);
   a.lut = device_lut(mask_table, lut);
   a.sync = sync;
   a.packets = reinterpret_cast<ulonglong2*>(sync + 4);
-  int f = 0;
-  auto field = [&](float* s0, float* s1) {
-    a.cur[f] = a.even[f] = s0;
-    a.prev[f] = a.odd[f] = s1;
-    ++f;
-  };
-  field(psi_r_s0, psi_r_s1);
-  if (cx) field(psi_i_s0, psi_i_s1);
-  field(chi_s0, chi_s1);
   e = lfm::launch_resident(a, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "resident run launch");
   return LFM_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int lfm_leapfrog_run_f32(int level, int steps, float* psi_r_s0, float* psi_r_s1,
+                         float* psi_i_s0, float* psi_i_s1, float* chi_s0, float* chi_s1,
+                         const float* mask_table, const lfm_mask_lut* lut, int damp_prev, int N,
+                         double dt2, double kappa, double lambda_self, double chi0, double e0_sq,
+                         double epsilon_w, float* const* stores, unsigned int* sync,
+                         void* stream) {
+  int rc = check_n(N);
+  if (rc) return rc;
+  const bool cx = level == LFM_COMPLEX;
+  float* const s0[3] = {psi_r_s0, psi_i_s0, chi_s0};
+  float* const s1[3] = {psi_r_s1, psi_i_s1, chi_s1};
+  const size_t b = sizeof(float) * (size_t)N * N * N;
+  std::vector<Span> slots = {{psi_r_s0, b}, {psi_r_s1, b}, {chi_s0, b}, {chi_s1, b}};
+  if (cx) {
+    slots.push_back({psi_i_s0, b});
+    slots.push_back({psi_i_s1, b});
+  }
+  rc = check_disjoint({}, slots);
+  if (rc) return rc;
+  return run_on_chip(level, steps, s0, s1, s0, s1, stores, mask_table, lut, damp_prev, N, dt2,
+                     kappa, lambda_self, chi0, e0_sq, epsilon_w, sync, stream);
+}
+
+int lfm_advance_run_f32(int level, int steps, const float* psi_r, const float* psi_r_prev,
+                        const float* psi_i, const float* psi_i_prev, const float* chi,
+                        const float* chi_prev, float* const* stores, const float* mask_table,
+                        const lfm_mask_lut* lut, int damp_prev, int N, double dt2, double kappa,
+                        double lambda_self, double chi0, double e0_sq, double epsilon_w,
+                        unsigned int* sync, void* stream) {
+  if (!stores) return fail(LFM_ERR_INVALID_ARG, "null buffer");
+  const float* const cur[3] = {psi_r, psi_i, chi};
+  const float* const prev[3] = {psi_r_prev, psi_i_prev, chi_prev};
+  return run_on_chip(level, steps, cur, prev, nullptr, nullptr, stores, mask_table, lut,
+                     damp_prev, N, dt2, kappa, lambda_self, chi0, e0_sq, epsilon_w, sync, stream);
 }
 
 int lfm_poisson_chi_f32(lfm_context* ctx, int level, const float* psi_r, const float* psi_i,

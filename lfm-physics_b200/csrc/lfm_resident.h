@@ -28,13 +28,16 @@ struct ResidentArgs {
   int level, N;
   int steps, damp_first;
   ResidentPlan plan;
-  // Psi_r, (Psi_i,) chi at the current time level and the one before; time
-  // levels of even / odd distance from the current one are stored to even /
-  // odd (for the two-slot layout: even = cur, odd = prev).
+  // Psi_r, (Psi_i,) chi at the current time level and the one before.  The last
+  // two time levels go to even / odd by their distance from the current one (the
+  // two-slot layout: even = cur, odd = prev), unless null; the level that step s
+  // makes also goes to stores[s * fields + f] (device memory), where stores and
+  // the entry are not null.
   const float* cur[3];
   const float* prev[3];
   float* even[3];
   float* odd[3];
+  float* const* stores;
   StepConsts c;
   MaskLut lut;
   uint32_t* sync;        // workspace words 0 (time base) and 1 (retired CTAs)

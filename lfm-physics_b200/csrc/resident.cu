@@ -164,10 +164,15 @@ struct Step {
   int cur;         // shared-memory slot of the current time level
   int to_prev;     // from a cell of the current slot to the other one's
   bool damp;       // previous Psi is stored undamped
-  bool store;      // one of the last two time levels: to the field slots
+  bool store;      // the new time level goes to global memory (s_dst)
   uint32_t t;      // the new time level
   ulonglong2* out; // the block's outer rows of time t in the exchange buffer
-  float* dst[3];
+};
+
+// Where a time level's fields go in global memory: the field slot (the last two time
+// levels) and the caller's store for that level, null = nowhere.
+struct Destinations {
+  float* p[2][3];
 };
 
 // The place of outer row (ii, jr) of an ni x nj block among its exchanged rows.
@@ -222,7 +227,8 @@ template <int LEVEL, bool EVEN, int PA, int PB, int PC>
 __device__ __forceinline__ void plane(const StepConsts& c, float* sm, const Block& B,
                                       const Cells& T, const Step& S,
                                       QPlane<kCells> (&Q)[kFields<LEVEL>][3], int ii,
-                                      RowOff& centre, RowWalk& walk, int& mask_at) {
+                                      RowOff& centre, RowWalk& walk, int& mask_at,
+                                      const Destinations& D) {
   constexpr int NS = kFields<LEVEL>, FS = kFieldFloats<LEVEL>, V = kCells;
   const RowOff nxt = ii + 1 < B.ni ? walk.next : halo_plane(B, T, true);
   step_rows(walk);
@@ -288,7 +294,10 @@ __device__ __forceinline__ void plane(const StepConsts& c, float* sm, const Bloc
   if (S.store) {
     const int g = ((B.i0 + ii) * B.N + B.j0 + T.jr) * B.N + T.k0;
 #pragma unroll
-    for (int f = 0; f < NS; ++f) store_global<EVEN>(S.dst[f] + g, out[f], T);
+    for (int f = 0; f < NS; ++f) {
+      if (D.p[0][f]) store_global<EVEN>(D.p[0][f] + g, out[f], T);
+      if (D.p[1][f]) store_global<EVEN>(D.p[1][f] + g, out[f], T);
+    }
   }
   centre = nxt;
 }
@@ -364,18 +373,58 @@ __device__ __forceinline__ bool receive(float* sm, const Block& B, const Cells& 
 
 // Copies rows listed in `rows` (global row numbers, -1 = none) of one array into
 // shared memory, row r at dst + 4 + r * RS, with the copies beyond its ends.  A warp
-// takes a row.
+// takes a row, eight rows' loads in flight (one at a time, filling a block of COMPLEX
+// 96^3 took 50 us).
 __device__ __forceinline__ void copy_rows(const float* src, float* dst, const int* rows,
                                           int count, const Block& B, int warp, int nwarps,
                                           int lane) {
-  for (int r = warp; r < count; r += nwarps) {
-    if (rows[r] < 0) continue;
-    const float* s = src + rows[r] * B.N;
-    float* d = dst + 4 + r * B.RS;
-    for (int k = lane; k < B.N; k += 32) d[k] = s[k];
-    if (lane == 0) {
-      d[B.N] = s[0];
-      d[-1] = s[B.N - 1];
+  constexpr int U = 8;
+  if ((B.N & 3) == 0) {
+    const int n4 = B.N >> 2;  // at most 32
+    for (int r = warp; r < count; r += U * nwarps) {
+      float4 t[U];
+      bool have[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int q = r + u * nwarps;
+        have[u] = q < count && lane < n4 && rows[q] >= 0;
+        if (have[u]) t[u] = *(reinterpret_cast<const float4*>(src + rows[q] * B.N) + lane);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (!have[u]) continue;
+        float* d = dst + 4 + (r + u * nwarps) * B.RS;
+        reinterpret_cast<float4*>(d)[lane] = t[u];
+        if (lane == 0) d[B.N] = t[u].x;
+        if (lane == n4 - 1) d[-1] = t[u].w;
+      }
+    }
+  } else {
+    for (int r = warp; r < count; r += U / 4 * nwarps) {
+      float t[U / 4][4];
+#pragma unroll
+      for (int u = 0; u < U / 4; ++u) {
+        const int q = r + u * nwarps;
+        if (q >= count || rows[q] < 0) continue;
+        const float* s = src + rows[q] * B.N;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (lane + 32 * k < B.N) t[u][k] = s[lane + 32 * k];
+      }
+#pragma unroll
+      for (int u = 0; u < U / 4; ++u) {
+        const int q = r + u * nwarps;
+        if (q >= count || rows[q] < 0) continue;
+        float* d = dst + 4 + q * B.RS;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int c = lane + 32 * k;
+          if (c >= B.N) continue;
+          d[c] = t[u][k];
+          if (c == 0) d[B.N] = t[u][k];
+          if (c == B.N - 1) d[-1] = t[u][k];
+        }
+      }
     }
   }
 }
@@ -386,6 +435,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   constexpr int V = kCells, NS = kFields<LEVEL>;
   extern __shared__ __align__(16) float sm[];
   __shared__ int s_abort;
+  __shared__ Destinations s_dst;
   const ResidentPlan& L = A.plan;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
   const int b = blockIdx.x, bi = b / L.nbj, bj = b % L.nbj;
@@ -453,11 +503,12 @@ __global__ void __launch_bounds__(THREADS, 1)
     copy_rows(A.prev[f], d + B.SLOT, own_row, L.NI * L.NJ, B, warp, nwarps, lane);
     copy_rows(A.cur[f], d + 2 * B.SLOT, halo_row, HR, B, warp, nwarps, lane);
   }
-  for (int r = warp; r < L.NI * L.NJ; r += nwarps) {
-    const int ii = r / L.NJ, jj = r % L.NJ;
-    const int q = qterm(B.i0 + ii, A.N) + qterm(B.j0 + jj, A.N);
-    for (int k = lane; k < B.N4; k += 32)
-      mask_rows[r * B.N4 + k] = mask_from_q_flat(A.lut, q + qterm(k < A.N ? k : 0, A.N));
+#pragma unroll 4
+  for (int x = tid; x < L.NI * L.NJ * B.N4; x += blockDim.x) {
+    const int r = x / B.N4, k = x - r * B.N4;
+    mask_rows[x] = mask_from_q_flat(A.lut, qterm(B.i0 + r / L.NJ, A.N) +
+                                               qterm(B.j0 + r % L.NJ, A.N) +
+                                               qterm(k < A.N ? k : 0, A.N));
   }
 
   Cells T;
@@ -476,6 +527,18 @@ __global__ void __launch_bounds__(THREADS, 1)
   const int rows_a_round = blockDim.x / groups;
   const int first_row = tid / groups < rows_a_round ? tid / groups : HR;
   const int64_t buffer = (int64_t)gridDim.x * OR * NP * groups;  // packets of one time level
+  // one thread a destination of the time level that step s makes
+  const auto set_destination = [&](int s) {
+    if (tid >= 2 * NS) return;
+    const int f = tid % NS;
+    float* p = nullptr;
+    if (tid < NS)
+      p = s >= A.steps - 2 ? ((s & 1) ? A.even[f] : A.odd[f]) : nullptr;
+    else if (A.stores)
+      p = A.stores[s * NS + f];
+    s_dst.p[tid / NS][f] = p;
+  };
+  set_destination(0);
   __syncthreads();
 
   // ---- steps ----------------------------------------------------------------
@@ -484,12 +547,10 @@ __global__ void __launch_bounds__(THREADS, 1)
     S.cur = s & 1;
     S.to_prev = (1 - 2 * S.cur) * B.SLOT;
     S.damp = s > 0 || A.damp_first;
-    S.store = s >= A.steps - 2;
+    S.store = s_dst.p[0][0] != nullptr || s_dst.p[1][0] != nullptr;
     S.t = base + (uint32_t)(s + 1);
     ulonglong2* packets = A.packets + (S.t & 1u) * buffer;
     S.out = packets + (int64_t)b * OR * NP * groups;
-#pragma unroll
-    for (int f = 0; f < NS; ++f) S.dst[f] = (s & 1) ? A.even[f] : A.odd[f];
     if (T.pa < T.pb) {
       QPlane<V> Q[NS][3];
       RowWalk walk = walk_from(B, T, S.cur, T.pa > 0 ? T.pa - 1 : 0);
@@ -501,11 +562,11 @@ __global__ void __launch_bounds__(THREADS, 1)
       for (int f = 0; f < NS; ++f) load_rows<V>(Q[f][1], sm + f * FS, centre);
       int ii = T.pa, mask_at = (T.pa * B.NJ + T.jr) * B.N4 + T.k0;
       while (true) {
-        plane<LEVEL, EVEN, 0, 1, 2>(A.c, sm, B, T, S, Q, ii, centre, walk, mask_at);
+        plane<LEVEL, EVEN, 0, 1, 2>(A.c, sm, B, T, S, Q, ii, centre, walk, mask_at, s_dst);
         if (++ii >= T.pb) break;
-        plane<LEVEL, EVEN, 1, 2, 0>(A.c, sm, B, T, S, Q, ii, centre, walk, mask_at);
+        plane<LEVEL, EVEN, 1, 2, 0>(A.c, sm, B, T, S, Q, ii, centre, walk, mask_at, s_dst);
         if (++ii >= T.pb) break;
-        plane<LEVEL, EVEN, 2, 0, 1>(A.c, sm, B, T, S, Q, ii, centre, walk, mask_at);
+        plane<LEVEL, EVEN, 2, 0, 1>(A.c, sm, B, T, S, Q, ii, centre, walk, mask_at, s_dst);
         if (++ii >= T.pb) break;
       }
     }
@@ -514,6 +575,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       s_abort = 1;
       atomicOr(A.status, LFM_ERR_DEVICE_TIMEOUT);
     }
+    set_destination(s + 1);  // behind receive()'s barrier: step s has stored
     __syncthreads();
     if (s_abort) break;
   }

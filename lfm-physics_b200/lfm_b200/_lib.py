@@ -72,6 +72,8 @@ _SIGNATURES = {
     "lfm_leapfrog_real_f32": [_P] * 5 + [POINTER(MaskLut), c_int, c_int] + [_D] * 5 + [_P],
     "lfm_leapfrog_complex_f32": [_P] * 7 + [POINTER(MaskLut), c_int, c_int] + [_D] * 6 + [_P],
     "lfm_leapfrog_run_f32": [c_int, c_int] + [_P] * 7 + [POINTER(MaskLut), c_int, c_int]
+    + [_D] * 6 + [_P, _P, _P],
+    "lfm_advance_run_f32": [c_int, c_int] + [_P] * 8 + [POINTER(MaskLut), c_int, c_int]
     + [_D] * 6 + [_P, _P],
     "lfm_leapfrog_run_words": [c_int, c_int, POINTER(ctypes.c_longlong)],
     "lfm_leapfrog_run_plan": [c_int, c_int, c_int, POINTER(c_int)],
@@ -169,13 +171,14 @@ def run_workspace(level: int, N: int, device):
     return torch.zeros(n.value, dtype=torch.int32, device=device)
 
 
-def run_steps(*args) -> bool:
-    """lfm_leapfrog_run_f32: True if the steps were launched, False if the lattice
-    has to take single steps (LFM_ERR_UNSUPPORTED); raises on any other error."""
-    rc = load().lfm_leapfrog_run_f32(*args)
+def run_steps(name: str, *args) -> bool:
+    """An on-chip run (lfm_leapfrog_run_f32, lfm_advance_run_f32): True if it was launched,
+    False if the lattice has to take single steps (LFM_ERR_UNSUPPORTED); raises on any
+    other error."""
+    rc = getattr(load(), name)(*args)
     if rc == LFM_ERR_UNSUPPORTED:
         return False
-    check(rc, "lfm_leapfrog_run_f32")
+    check(rc, name)
     return True
 
 

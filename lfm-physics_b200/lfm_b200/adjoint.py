@@ -34,6 +34,8 @@ FIELDS = ("psi_r", "psi_r_prev", "psi_i", "psi_i_prev", "chi", "chi_prev")
 class _Lattice:
     """Resident slots of one lattice plus the calls that step and un-step it."""
 
+    on_chip = True  # its steps may run on chip
+
     def __init__(self, config, backend: B200Backend) -> None:
         self.config = config
         self.backend = backend
@@ -54,6 +56,7 @@ class _Lattice:
         self.chi = [torch.empty(self.n, **f32) for _ in range(2)]
         self.cur = 0
         self.damp = False
+        self.run_sync = None  # workspace of the on-chip runs, made on first use
         c = config
         self.common = (float(c.dt) ** 2, float(c.kappa), float(c.lambda_self), float(c.chi0),
                        float(c.e0_sq))
@@ -106,6 +109,47 @@ class _Lattice:
                       self.N, *self.common, stream)
         self.cur = p
         self.damp = True
+
+    def _run(self, name: str, steps: int, fields, stores, damp: bool) -> bool:
+        if self.run_sync is None:
+            self.run_sync = _lib.run_workspace(int(self.level), self.N, self.device)
+        if self.run_sync.numel() == 0:
+            return False
+        ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
+        order = [ptr(t) for t in fields]
+        tail = (self.table.data_ptr(), ctypes.byref(self.desc), int(damp), self.N, *self.common,
+                float(self.config.epsilon_w))
+        where = (ptr(stores),)
+        end = (self.run_sync.data_ptr(), _stream_handle(self.device))
+        if name == "lfm_advance_run_f32":
+            return _lib.run_steps(name, int(self.level), steps, *order, *where, *tail, *end)
+        return _lib.run_steps(name, int(self.level), steps, *order, *tail, *where, *end)
+
+    def run(self, steps: int, stores=None) -> bool:
+        """`steps` steps in place with the state held on chip (lfm_leapfrog_run_f32), the
+        time levels listed in `stores` (store_table) stored on the way; False, with
+        nothing done, if the lattice has to take single steps."""
+        c, p = self.cur, 1 - self.cur
+        pi = (self.pi[c], self.pi[p]) if self.cx else (None, None)
+        if not self._run("lfm_leapfrog_run_f32", steps,
+                         (self.pr[c], self.pr[p], *pi, self.chi[c], self.chi[p]), stores,
+                         self.damp):
+            return False
+        self.cur = p if steps % 2 else c
+        self.damp = True
+        return True
+
+    def advance_run(self, cur, prev, steps: int, stores, damp: bool) -> bool:
+        """The same out of place from (psi_r, psi_i, chi) triples (lfm_advance_run_f32)."""
+        return self._run("lfm_advance_run_f32", steps,
+                         (cur[0], prev[0], cur[1], prev[1], cur[2], prev[2]), stores, damp)
+
+    def store_table(self, levels):
+        """Device table of the buffers that the time levels of an on-chip run go to: one
+        state buffer or None per step."""
+        rows = [[0] * (3 if self.cx else 2) if st is None
+                else [t.data_ptr() for t in st if t is not None] for st in levels]
+        return torch.tensor(rows, dtype=torch.int64).to(self.device)
 
     def advance(self, cur, prev, out, damp: bool) -> None:
         """One step out of place: cur / prev / out are (psi_r, psi_i, chi) triples
@@ -196,6 +240,11 @@ class _SplitLattice(_Lattice):
                       prev_io[3].data_ptr(), tab, desc, int(damp), self.N, *self.common,
                       stream)
 
+    on_chip = False  # split chi takes single steps
+
+    def _run(self, *args) -> bool:
+        return False
+
     def step(self) -> None:
         c, p = self.cur, 1 - self.cur
         self._split_step(self.slots(c), self.slots(p), self.damp)
@@ -237,20 +286,38 @@ class _Plan:
         self.bwd_graph = None
         self.busy = False
 
+        # on-chip runs store the checkpoints and the segment's states as they pass: time
+        # level t is checkpoint t / every's current state, t + 1 a multiple's previous one
+        # (with every = 1 a level is both: single steps)
+        self.fwd_stores = self.seg_stores = None
+        if every > 1 and lat.on_chip:
+            marks = {}
+            for k in range(1, len(self.snaps)):
+                marks[k * every], marks[k * every - 1] = self.snaps[k]
+            self.fwd_stores = lat.store_table([marks.get(t + 1) for t in range(steps)])
+            self.seg_stores = lat.store_table(self.seg)
+
     # ---- bodies (run eagerly or under capture) ----
+    def _checkpoint(self, k: int) -> None:
+        lat = self.lat
+        cur, prev = self.snaps[k]
+        c, p = lat.cur, 1 - lat.cur
+        for dst, src in ((cur, lat.slots(c)), (prev, lat.slots(p))):
+            for d, x in zip(dst, src):
+                if d is not None:
+                    d.copy_(x)
+        self.meta[k] = lat.damp
+
     def forward_body(self) -> None:
         lat = self.lat
         lat.cur, lat.damp = 0, False
+        self._checkpoint(0)
+        if self.fwd_stores is not None and lat.run(self.steps, self.fwd_stores):
+            self.meta[1:] = [True] * (len(self.meta) - 1)
+            return
         for t in range(self.steps):
-            if t % self.every == 0:
-                k = t // self.every
-                cur, prev = self.snaps[k]
-                c, p = lat.cur, 1 - lat.cur
-                for dst, src in ((cur, lat.slots(c)), (prev, lat.slots(p))):
-                    for d, x in zip(dst, src):
-                        if d is not None:
-                            d.copy_(x)
-                self.meta[k] = lat.damp
+            if t and t % self.every == 0:
+                self._checkpoint(t // self.every)
             lat.step()
 
     def backward_body(self) -> int:
@@ -265,10 +332,12 @@ class _Plan:
             e0 = min(s0 + every, steps)
             c0, p0 = self.snaps[si]
             states = [c0] + self.seg[: e0 - s0]
-            for t in range(s0, e0):
-                u = t - s0
-                lat.advance(states[u], p0 if u == 0 else states[u - 1], states[u + 1],
-                            self.meta[si] if u == 0 else True)
+            if not (self.seg_stores is not None and e0 - s0 > 1
+                    and lat.advance_run(c0, p0, e0 - s0, self.seg_stores, self.meta[si])):
+                for t in range(s0, e0):
+                    u = t - s0
+                    lat.advance(states[u], p0 if u == 0 else states[u - 1], states[u + 1],
+                                self.meta[si] if u == 0 else True)
             for t in range(e0 - 1, s0 - 1, -1):
                 lat.adjoint_step(states[t - s0], states[t - s0 + 1], self.g[cur],
                                  self.g[1 - cur])
@@ -390,8 +459,9 @@ def leapfrog(config, state, steps: int, every: int | None = None, backend="auto"
         s is not None and s.requires_grad for s in state)
     if not needs_grad:
         lat.load(state)
-        for _ in range(steps):
-            lat.step()
+        if steps < 2 or not lat.run(steps):
+            for _ in range(steps):
+                lat.step()
         return tuple(None if o is None else o.reshape(lat.N, lat.N, lat.N) for o in lat.state())
     return LeapfrogFunction.apply(_plan_for(lat, steps, every), *state)
 

@@ -361,11 +361,12 @@ class Evolver:
         pi = ((self._pi[cur].data_ptr(), self._pi[prv].data_ptr()) if self._has_imag
               else (None, None))
         if not _lib.run_steps(
-                int(self._level), steps, self._pr[cur].data_ptr(), self._pr[prv].data_ptr(), *pi,
+                "lfm_leapfrog_run_f32", int(self._level), steps, self._pr[cur].data_ptr(), self._pr[prv].data_ptr(), *pi,
                 self._chi[cur].data_ptr(), self._chi[prv].data_ptr(), self._table_dev.data_ptr(),
                 ctypes.byref(self._desc), 1 if self._damp else 0, self.N, float(self._dt2),
                 float(cfg.kappa), float(cfg.lambda_self), float(cfg.chi0), float(cfg.e0_sq),
-                float(cfg.epsilon_w), self._run_sync.data_ptr(), _stream_handle(self.device)):
+                float(cfg.epsilon_w), None, self._run_sync.data_ptr(),
+                _stream_handle(self.device)):
             return False
         if steps % 2:
             self._cur = prv
