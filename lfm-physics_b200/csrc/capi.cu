@@ -250,24 +250,49 @@ int poisson_slot(lfm_context* ctx, int N, PoissonSlot** out) {
   return LFM_OK;
 }
 
+bool capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+}
+
+// The filter table for (gamma, D), made on first use (outside stream capture: it
+// allocates).
+int filter_table(FftSlot* s, int N, double gamma, double d, cudaStream_t stream, float** table) {
+  const std::pair<double, double> key(gamma, d);
+  auto it = s->tables.find(key);
+  if (it != s->tables.end()) {
+    *table = it->second;
+    return LFM_OK;
+  }
+  const size_t nz = N / 2 + 1;
+  float* t = nullptr;
+  cudaError_t e = cudaMalloc(&t, sizeof(float) * nz * nz * nz);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc filter table");
+  e = lfm::launch_helmholtz_table(t, N, gamma, d, stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+  if (e != cudaSuccess) {
+    cudaFree(t);
+    return cuda_fail(e, "filter table");
+  }
+  s->tables[key] = t;
+  *table = t;
+  return LFM_OK;
+}
+
 // The split transform's plans, twiddles and the filter table for (gamma, D),
 // created on first use (outside stream capture: they allocate and upload).
 int split_transform(FftSlot* s, int N, double gamma, double d, cudaStream_t stream,
                     float** table) {
-  const std::pair<double, double> key(gamma, d);
-  auto it = s->tables.find(key);
-  if (s->r2c_2d && it != s->tables.end()) {
-    *table = it->second;
+  if (s->r2c_2d && s->tables.count({gamma, d})) {
+    *table = s->tables[{gamma, d}];
     return LFM_OK;
   }
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  cudaError_t e = cudaStreamIsCapturing(stream, &cap);
-  if (e != cudaSuccess) return cuda_fail(e, "cudaStreamIsCapturing");
-  if (cap != cudaStreamCaptureStatusNone)
+  if (capturing(stream))
     return fail(LFM_ERR_UNSUPPORTED,
                 "the first S_a solve for N=%d, gamma=%g, D=%g must run outside stream capture",
                 N, gamma, d);
   const int nz = N / 2 + 1;
+  cudaError_t e = cudaSuccess;
   if (!s->r2c_2d) {
     int n[2] = {N, N}, inr[2] = {N, N}, inc[2] = {N, nz};
     if (cufftPlanMany(&s->r2c_2d, 2, n, inr, 1, N * N, inc, 1, N * nz, CUFFT_R2C, 3 * N) !=
@@ -287,18 +312,7 @@ int split_transform(FftSlot* s, int N, double gamma, double d, cudaStream_t stre
     if (e == cudaSuccess) e = lfm::upload_dft_twiddles();  // this context's device
     if (e != cudaSuccess) return cuda_fail(e, "twiddle table");
   }
-  float* t = nullptr;
-  e = cudaMalloc(&t, sizeof(float) * (size_t)nz * nz * nz);
-  if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc filter table");
-  e = lfm::launch_helmholtz_table(t, N, gamma, d, stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-  if (e != cudaSuccess) {
-    cudaFree(t);
-    return cuda_fail(e, "filter table");
-  }
-  s->tables[key] = t;
-  *table = t;
-  return LFM_OK;
+  return filter_table(s, N, gamma, d, stream, table);
 }
 
 // S_a from |Psi_a|^2: from pr, pi (the energy is formed first, into the
@@ -338,7 +352,17 @@ int helmholtz(lfm_context* ctx, const float* pr, const float* pi, float* sa_raw,
       cufftExecR2C(s->r2c, const_cast<float*>(src),
                    reinterpret_cast<cufftComplex*>(s->spec)) != CUFFT_SUCCESS)
     return fail(LFM_ERR_CUFFT, "cufftExecR2C N=%d", N);
-  e = lfm::launch_helmholtz_multiply_gd(s->spec, N, gamma, d, stream);
+  // The factors from a table (a float64 division, three 64-bit divisions a point
+  // otherwise); a solve with new constants under capture, which may not allocate,
+  // works them out.
+  if (s->tables.count({gamma, d}) || !capturing(stream)) {
+    float* table = nullptr;
+    rc = filter_table(s, N, gamma, d, stream, &table);
+    if (rc) return rc;
+    e = lfm::launch_helmholtz_multiply_table(s->spec, N, table, stream);
+  } else {
+    e = lfm::launch_helmholtz_multiply_gd(s->spec, N, gamma, d, stream);
+  }
   if (e != cudaSuccess) return cuda_fail(e, "Helmholtz multiply launch");
   if (cufftSetStream(s->c2r, stream) != CUFFT_SUCCESS ||
       cufftExecC2R(s->c2r, reinterpret_cast<cufftComplex*>(s->spec), dst) != CUFFT_SUCCESS)

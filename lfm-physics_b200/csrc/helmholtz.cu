@@ -4,6 +4,8 @@
 // (lfm/core/backends/numpy_backend.py:341-356).  The filter is evaluated in
 // float64 from k = 2*pi*fftfreq(N) exactly as NumPy builds it, divided by
 // N^3 (cuFFT's inverse is unnormalised) and applied in float32.
+#include <algorithm>
+
 #include "lfm_kernels.h"
 
 namespace lfm {
@@ -68,6 +70,27 @@ __global__ void helmholtz_multiply_kernel(float2* __restrict__ spec, int N, doub
   }
 }
 
+// The same multiplication with the factors from the table of helmholtz_table_kernel
+// (spectral.cu; the same float64 operations, rounded once): blockIdx.y is x, the
+// threads run over a plane's (y, z).
+__global__ void helmholtz_multiply_table_kernel(float2* __restrict__ spec, int N,
+                                                const float* __restrict__ table) {
+  const int H = N / 2 + 1, plane = N * H;
+  const int x = blockIdx.y, fx = x <= N - x ? x : N - x;
+  const int64_t per_colour = (int64_t)N * plane;
+  for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < plane; w += gridDim.x * blockDim.x) {
+    const int y = w / H, z = w - y * H, fy = y <= N - y ? y : N - y;
+    const float scale = __ldg(table + ((int64_t)fx * H + fy) * H + z);
+    float2* p = spec + (int64_t)x * plane + w;
+    float2 v[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) v[a] = p[a * per_colour];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+      p[a * per_colour] = make_float2(v[a].x * scale, v[a].y * scale);
+  }
+}
+
 __global__ void clip_kernel(const float* __restrict__ in, float* __restrict__ out, int64_t n) {
   for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < n;
        x += (int64_t)gridDim.x * blockDim.x)
@@ -102,6 +125,14 @@ cudaError_t launch_helmholtz_multiply_gd(float2* spec, int N, double gamma, doub
   const int64_t per_colour = (int64_t)N * N * (N / 2 + 1);
   helmholtz_multiply_kernel<<<grid_for(per_colour, 256), 256, 0, stream>>>(spec, N, gamma, d,
                                                                            per_colour);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_helmholtz_multiply_table(float2* spec, int N, const float* table,
+                                            cudaStream_t stream) {
+  const int plane = N * (N / 2 + 1);
+  const dim3 grid((unsigned)std::min((plane + 255) / 256, 64), (unsigned)N);
+  helmholtz_multiply_table_kernel<<<grid, 256, 0, stream>>>(spec, N, table);
   return cudaGetLastError();
 }
 

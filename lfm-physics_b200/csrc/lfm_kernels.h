@@ -70,6 +70,9 @@ cudaError_t launch_color_energy(const float* pr, const float* pi, float* e, int 
                                 cudaStream_t stream);
 cudaError_t launch_helmholtz_multiply_gd(float2* spec, int N, double gamma, double d,
                                          cudaStream_t stream);
+// ... and with the factors from launch_helmholtz_table's table.
+cudaError_t launch_helmholtz_multiply_table(float2* spec, int N, const float* table,
+                                            cudaStream_t stream);
 cudaError_t launch_clip(const float* in, float* out, int64_t count, cudaStream_t stream);
 // The split S_a transform (spectral.cu): which N it serves, the filter table
 // ((N/2+1)^3 floats) and the fused pass along i on spec[3][N][N*(N/2+1)].

@@ -285,11 +285,12 @@ __device__ __forceinline__ void field_stencil(const float* smem, int fm, int f0,
 
 // One output plane of the COLOR step: seven 19-point stencils from the
 // ring, the point fields from global memory, lfm_cells.cuh's colour update.
-template <int V>
+template <int V, class G>
 __device__ __forceinline__ void color_plane(const TmaParams& P, const float* smem, int sm, int s0,
                                             int sp, int i, const Lane& L, int j) {
   const StepArgs& a = P.a;
-  const int N = P.N, TJ = P.TJ;
+  const G geo(P);
+  const int N = geo.N, TJ = geo.TJ;
   const int field_rows = (TJ + 2) * N;
   const int64_t gofs = ((int64_t)i * N + j) * N + L.k0;
 
@@ -507,14 +508,30 @@ __device__ __forceinline__ void issue_plane(const TmaParams& P, float* smem, uin
 template <int LEVEL, int MODE>
 constexpr bool kOneCopy = LEVEL == LFM_COMPLEX || MODE != kPlain;
 
-template <int LEVEL, int V>
-__global__ void __launch_bounds__(512) tma_step_kernel(const __grid_constant__ TmaParams P) {
+// Geometry of the barrier kernel's tile: from the parameters, or fixed.
+struct ColorRT {
+  static constexpr int kThreads = 512, kCtas = 1;
+  int N, TJ, S, SF;
+  __device__ __forceinline__ explicit ColorRT(const TmaParams& P)
+      : N(P.N), TJ(P.TJ), S(P.S), SF(P.stage_floats) {}
+};
+template <int N_, int TJ_, int S_>
+struct ColorCT {
+  static constexpr int kThreads = TJ_ * N_ / 2, kCtas = 512 / kThreads;
+  static constexpr int N = N_, TJ = TJ_, S = S_, SF = N_ * 7 * (TJ_ + 2);
+  __device__ __forceinline__ explicit ColorCT(const TmaParams&) {}
+};
+
+template <int LEVEL, int V, class G = ColorRT>
+__global__ void __launch_bounds__(G::kThreads, G::kCtas)
+    tma_step_kernel(const __grid_constant__ TmaParams P) {
   static_assert(LEVEL == LFM_COLOR, "REAL and COMPLEX run on the register-queue kernel");
   extern __shared__ __align__(128) float smem[];
   __shared__ __align__(8) uint64_t bars[kMaxStages];
   __shared__ int abort_flag;
 
-  const int N = P.N, TJ = P.TJ, S = P.S;
+  const G geo(P);
+  const int N = geo.N, TJ = geo.TJ, S = geo.S;
   const int jt = blockIdx.x % P.JT, ch = blockIdx.x / P.JT;
   const int j0 = jt * TJ;
   const int i0 = ch * P.IC;
@@ -556,8 +573,8 @@ __global__ void __launch_bounds__(512) tma_step_kernel(const __grid_constant__ T
       abort_flag = 1;
       atomicOr(P.a.status, LFM_ERR_DEVICE_TIMEOUT);
     } else {
-      const int sf = P.stage_floats;
-      color_plane<V>(P, smem, (c % S) * sf, ((c + 1) % S) * sf, ((c + 2) % S) * sf,
+      const int sf = geo.SF;
+      color_plane<V, G>(P, smem, (c % S) * sf, ((c + 1) % S) * sf, ((c + 2) % S) * sf,
                               i0 + c, L, j);
     }
     __syncthreads();
@@ -1536,6 +1553,22 @@ bool try_fixed(TmaParams& P, const Choice& ch, cudaStream_t stream, cudaError_t*
   return false;
 }
 
+// The barrier kernel's compile-time tiles.
+template <int N, int TJ, int S>
+cudaError_t launch_color(TmaParams& P, const Choice& ch, cudaStream_t stream) {
+  static std::mutex mu;
+  static int granted = 0;
+  return launch_kernel(tma_step_kernel<LFM_COLOR, 2, ColorCT<N, TJ, S>>, &granted, &mu, P, ch,
+                       stream);
+}
+
+bool try_color(TmaParams& P, const Choice& ch, cudaStream_t stream, cudaError_t* err) {
+  if (P.N == 256 && ch.TJ == 2 && ch.S == 4) { *err = launch_color<256, 2, 4>(P, ch, stream); return true; }
+  if (P.N == 128 && ch.TJ == 4 && ch.S == 5) { *err = launch_color<128, 4, 5>(P, ch, stream); return true; }
+  if (P.N == 64 && ch.TJ == 8 && ch.S == 5) { *err = launch_color<64, 8, 5>(P, ch, stream); return true; }
+  return false;
+}
+
 template <int LEVEL, int V, bool QUEUE, int MODE = kPlain>
 cudaError_t plan_and_launch(TmaParams& P, const TileConfig* forced, cudaStream_t stream) {
   using Slot = KernelSlot<LEVEL, V, QUEUE, MODE>;
@@ -1588,6 +1621,10 @@ cudaError_t plan_and_launch(TmaParams& P, const TileConfig* forced, cudaStream_t
   if constexpr (QUEUE) {
     cudaError_t fe = cudaSuccess;
     if (try_fixed<LEVEL, V, MODE>(P, ch, stream, &fe)) return fe;
+  }
+  if constexpr (LEVEL == LFM_COLOR && V == 2) {
+    cudaError_t ce = cudaSuccess;
+    if (try_color(P, ch, stream, &ce)) return ce;
   }
   return launch_kernel(Slot::fn(), &Slot::granted, &Slot::mu, P, ch, stream);
 }
