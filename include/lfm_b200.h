@@ -402,6 +402,13 @@ typedef struct lfm_batch_tuning {
 
 typedef struct lfm_batch lfm_batch;
 
+/* `steps` steps of every lattice with the state held on chip, waves of lattices one
+ * after another (the same bits as `steps` calls of lfm_batch_step; the current fields
+ * are then in slot parity + steps mod 2).  LFM_ERR_UNSUPPORTED, with nothing launched,
+ * when a lattice does not fit on chip, steps < 2 or a step path is forced. */
+int lfm_batch_run(lfm_batch* batch, int steps, int parity, int damp_prev, void* stream);
+
+
 /* Plans the work lists and uploads the descriptors (device memory owned by
  * the batch).  tuning may be NULL.  The buffers stay owned by the caller. */
 int lfm_batch_create(const lfm_lattice_desc* lattices, int count,

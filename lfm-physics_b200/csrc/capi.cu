@@ -1493,6 +1493,10 @@ struct lfm_batch {
   int* d_counters = nullptr;  // next item of each shape class, then retired CTAs
   int nitems = 0, real_items = 0, threads = 0, smem = 0, grid = 0;
   int class_off[lfm::kBatchClasses] = {}, class_n[lfm::kBatchClasses] = {};
+  // on-chip runs (lfm_batch_run): the lattices, their waves and the waves' workspace
+  std::vector<lfm::BatchLattice> lat;
+  std::vector<lfm::ResidentWavePlan> waves;
+  uint32_t* d_sync = nullptr;
 };
 
 extern "C" {
@@ -1612,7 +1616,73 @@ int lfm_batch_create(const lfm_lattice_desc* lattices, int count,
     lfm_batch_destroy(B);
     return cuda_fail(e, "batch descriptors");
   }
+  // Waves of lattices held on chip, for lfm_batch_run.
+  std::vector<int> level(count), edge(count);
+  for (int l = 0; l < count; ++l) {
+    level[l] = dev[l].level;
+    edge[l] = dev[l].N;
+  }
+  double cycles = 0.0;
+  if (lfm::resident_waves(level.data(), edge.data(), count, sms, &B->waves, &cycles)) {
+    long long words = 0;
+    for (const lfm::ResidentWavePlan& w : B->waves) {
+      long long sum = 0;
+      for (const lfm::ResidentPlan& p : w.plans) sum += p.words;
+      words = std::max(words, sum);
+    }
+    e = cudaMalloc(&B->d_sync, 4 * (size_t)words);
+    if (e == cudaSuccess) e = cudaMemset(B->d_sync, 0, 4 * (size_t)words);
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e != cudaSuccess) {  // no memory for it: the lattices take single steps
+      cudaGetLastError();
+      if (B->d_sync) cudaFree(B->d_sync);
+      B->d_sync = nullptr;
+      B->waves.clear();
+    }
+  }
+  B->lat = std::move(dev);
   *out = B;
+  return LFM_OK;
+}
+
+int lfm_batch_run(lfm_batch* batch, int steps, int parity, int damp_prev, void* stream) {
+  if (!batch) return fail(LFM_ERR_INVALID_ARG, "null batch");
+  if (parity != 0 && parity != 1) return fail(LFM_ERR_INVALID_ARG, "parity %d", parity);
+  if (batch->waves.empty() || steps < 2)
+    return fail(LFM_ERR_UNSUPPORTED, "batch run: %d steps, %zu waves", steps, batch->waves.size());
+  if (g_path.load() != 0) return fail(LFM_ERR_UNSUPPORTED, "batch run: a step path is forced");
+  int* status = nullptr;
+  int rc = status_word(&status);
+  if (rc) return rc;
+  for (const lfm::ResidentWavePlan& w : batch->waves) {
+    std::vector<lfm::ResidentArgs> args(w.lattices.size());
+    uint32_t* at = batch->d_sync + 4;
+    for (size_t k = 0; k < args.size(); ++k) {
+      const lfm::BatchLattice& b = batch->lat[w.lattices[k]];
+      lfm::ResidentArgs& a = args[k];
+      a.level = b.level;
+      a.N = b.N;
+      a.steps = steps;
+      a.damp_first = damp_prev ? 1 : 0;
+      a.plan = w.plans[k];
+      int f = 0;
+      for (float* const* slot : {b.pr, b.pi, b.chi}) {
+        if (!slot[0]) continue;  // Psi_i at REAL
+        a.cur[f] = a.even[f] = slot[parity];
+        a.prev[f] = a.odd[f] = slot[1 - parity];
+        ++f;
+      }
+      a.c = b.c;
+      a.lut = b.lut;
+      a.sync = batch->d_sync;
+      a.packets = reinterpret_cast<ulonglong2*>(at);
+      at += w.plans[k].words - 4;
+      a.status = status;
+    }
+    cudaError_t e = lfm::launch_resident_wave(args.data(), (int)args.size(),
+                                              static_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return cuda_fail(e, "batch run launch");
+  }
   return LFM_OK;
 }
 
@@ -1661,6 +1731,7 @@ int lfm_batch_destroy(lfm_batch* batch) {
   if (batch->d_lat) cudaFree(batch->d_lat);
   if (batch->d_items) cudaFree(batch->d_items);
   if (batch->d_counters) cudaFree(batch->d_counters);
+  if (batch->d_sync) cudaFree(batch->d_sync);
   cudaSetDevice(prev);
   delete batch;
   return LFM_OK;

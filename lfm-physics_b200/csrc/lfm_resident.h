@@ -2,6 +2,8 @@
 #pragma once
 
 #include <cstdint>
+#include <vector>
+
 #include <cuda_runtime.h>
 
 #include "lfm_math.cuh"
@@ -18,6 +20,7 @@ struct ResidentPlan {
   int RS = 0;    // floats of a shared-memory row
   int smem = 0;  // bytes of dynamic shared memory
   long long words = 0;  // 32-bit words of the workspace: 4 counters, two exchange buffers
+  double cycles = 0;    // the model's time of a step
 };
 
 // The plan of an N^3 lattice at `level` on `sms` SMs; false if its state does
@@ -46,5 +49,21 @@ struct ResidentArgs {
 };
 
 cudaError_t launch_resident(const ResidentArgs& a, cudaStream_t stream);
+
+// Lattices of one level that run side by side in one launch, each on its own blocks.
+struct ResidentWavePlan {
+  int level, blocks;
+  std::vector<int> lattices;
+  std::vector<ResidentPlan> plans;
+};
+constexpr int kWaveLattices = 32;  // at most, in a wave
+
+// The waves that run `count` lattices on chip one wave after another, and the model's
+// cycles of a step through all of them; false if a lattice does not fit or its N is odd.
+bool resident_waves(const int* level, const int* N, int count, int sms,
+                    std::vector<ResidentWavePlan>* waves, double* cycles);
+
+// One wave: the same steps, sync and status for all; packets apart.
+cudaError_t launch_resident_wave(const ResidentArgs* a, int count, cudaStream_t stream);
 
 }  // namespace lfm

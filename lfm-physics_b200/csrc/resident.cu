@@ -27,10 +27,11 @@
 //
 // Arithmetic: lfm_cells.cuh in the order of the other kernels, bit-identical.
 #include <algorithm>
-#include <array>
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <utility>
+#include <vector>
 
 #include "lfm_kernels.h"
 #include "lfm_queue.cuh"
@@ -40,6 +41,8 @@ namespace lfm {
 namespace {
 
 constexpr int kMaxThreads = 512;
+constexpr int kThreadsComplex = 384;  // COMPLEX takes up to 168 registers
+constexpr int kMaxBlocks = 148;  // one block an SM
 // Cells a thread: two (one packed pair).  Four were slower at every REAL size (64^3
 // 3.99 against 3.53 us a step, 96^3 8.1 against 7.5): their k neighbours meet in
 // four-way bank conflicts, and half the threads are left to hide latency.
@@ -429,16 +432,28 @@ __device__ __forceinline__ void copy_rows(const float* src, float* dst, const in
   }
 }
 
-template <int LEVEL, bool EVEN, int THREADS>
+// The lattices of a launch: CTAs [first[l], first[l + 1]) run lattice l.
+template <int LATTICES>
+struct Wave {
+  int count;
+  int first[LATTICES + 1];
+  ResidentArgs lattice[LATTICES];
+};
+
+template <int LEVEL, bool EVEN, int THREADS, int LATTICES>
 __global__ void __launch_bounds__(THREADS, 1)
-    resident_kernel(const __grid_constant__ ResidentArgs A) {
+    resident_kernel(const __grid_constant__ Wave<LATTICES> W) {
   constexpr int V = kCells, NS = kFields<LEVEL>;
+  int l = 0;
+  if constexpr (LATTICES > 1)
+    while ((int)blockIdx.x >= W.first[l + 1]) ++l;
+  const ResidentArgs& A = W.lattice[l];
   extern __shared__ __align__(16) float sm[];
   __shared__ int s_abort;
   __shared__ Destinations s_dst;
   const ResidentPlan& L = A.plan;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-  const int b = blockIdx.x, bi = b / L.nbj, bj = b % L.nbj;
+  const int b = blockIdx.x - (LATTICES > 1 ? W.first[l] : 0), bi = b / L.nbj, bj = b % L.nbj;
   Block B;
   B.N = A.N;
   B.N4 = (A.N + 3) & ~3;
@@ -526,7 +541,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   T.pb = active ? (seg + 1) * B.ni / L.segs : 0;
   const int rows_a_round = blockDim.x / groups;
   const int first_row = tid / groups < rows_a_round ? tid / groups : HR;
-  const int64_t buffer = (int64_t)gridDim.x * OR * NP * groups;  // packets of one time level
+  const int64_t buffer = (int64_t)L.nbi * L.nbj * OR * NP * groups;  // packets of a time level
   // one thread a destination of the time level that step s makes
   const auto set_destination = [&](int s) {
     if (tid >= 2 * NS) return;
@@ -589,31 +604,57 @@ __global__ void __launch_bounds__(THREADS, 1)
   }
 }
 
-template <int LEVEL, bool EVEN, int THREADS>
-cudaError_t launch(const ResidentArgs& a, cudaStream_t stream) {
+template <int LEVEL, bool EVEN, int THREADS, int LATTICES>
+cudaError_t launch(const Wave<LATTICES>& w, int threads, int smem, cudaStream_t stream) {
   static std::mutex mu;
   static int granted = 0;
-  const auto kernel = resident_kernel<LEVEL, EVEN, THREADS>;
+  const auto kernel = resident_kernel<LEVEL, EVEN, THREADS, LATTICES>;
   {
     std::lock_guard<std::mutex> lk(mu);
-    if (a.plan.smem > granted) {
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           a.plan.smem);
+    if (smem > granted) {
+      cudaError_t e =
+          cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
       if (e != cudaSuccess) return e;
-      granted = a.plan.smem;
+      granted = smem;
     }
   }
-  void* args[] = {const_cast<ResidentArgs*>(&a)};
-  return cudaLaunchCooperativeKernel((const void*)kernel, dim3(a.plan.nbi * a.plan.nbj),
-                                     dim3(a.plan.threads), args, (size_t)a.plan.smem, stream);
+  void* args[] = {const_cast<Wave<LATTICES>*>(&w)};
+  return cudaLaunchCooperativeKernel((const void*)kernel, dim3(w.first[w.count]), dim3(threads),
+                                     args, (size_t)smem, stream);
 }
 
 template <int LEVEL>
 cudaError_t launch_level(const ResidentArgs& a, cudaStream_t stream) {
-  const bool small = a.plan.threads <= 384, even = a.N % 2 == 0;
-  if (even)
-    return small ? launch<LEVEL, true, 384>(a, stream) : launch<LEVEL, true, 512>(a, stream);
-  return small ? launch<LEVEL, false, 384>(a, stream) : launch<LEVEL, false, 512>(a, stream);
+  Wave<1> w{1, {0, a.plan.nbi * a.plan.nbj}, {a}};
+  const int t = a.plan.threads, sm = a.plan.smem;
+  if constexpr (LEVEL == LFM_COMPLEX)
+    return a.N % 2 == 0 ? launch<LEVEL, true, kThreadsComplex>(w, t, sm, stream)
+                        : launch<LEVEL, false, kThreadsComplex>(w, t, sm, stream);
+  else if (a.N % 2 == 0)
+    return t <= 384 ? launch<LEVEL, true, 384>(w, t, sm, stream)
+                    : launch<LEVEL, true, 512>(w, t, sm, stream);
+  else
+    return t <= 384 ? launch<LEVEL, false, 384>(w, t, sm, stream)
+                    : launch<LEVEL, false, 512>(w, t, sm, stream);
+}
+
+template <int LEVEL>
+cudaError_t launch_wave(const ResidentArgs* a, int count, cudaStream_t stream) {
+  static_assert(sizeof(Wave<kWaveLattices>) < 32000, "kernel parameters");
+  Wave<kWaveLattices> w{};
+  w.count = count;
+  int threads = 0, smem = 0;
+  for (int l = 0; l < count; ++l) {
+    w.lattice[l] = a[l];
+    w.first[l + 1] = w.first[l] + a[l].plan.nbi * a[l].plan.nbj;
+    threads = std::max(threads, a[l].plan.threads);
+    smem = std::max(smem, a[l].plan.smem);
+  }
+  if constexpr (LEVEL == LFM_COMPLEX)
+    return launch<LEVEL, true, kThreadsComplex>(w, threads, smem, stream);
+  else
+    return threads <= 384 ? launch<LEVEL, true, 384>(w, threads, smem, stream)
+                          : launch<LEVEL, true, 512>(w, threads, smem, stream);
 }
 
 }  // namespace
@@ -623,30 +664,25 @@ cudaError_t launch_level(const ResidentArgs& a, cudaStream_t stream) {
 // one warp's own latency), the halo packets a CTA reads, and the latency of the
 // exchange.  Measured on B200: a warp's plane 330 (REAL) / 480 (COMPLEX) cycles
 // with several warps on the scheduler, 900 / 1200 alone; 0.7 cycles a packet; 2300
-// for the exchange itself.  COMPLEX spills at 512 threads, hence the factor there.
+// for the exchange itself.
 // Best of the cuts tried, and this model's: REAL 32^3 2.16 / 2.23 us a step, 64^3
 // 3.53 / 3.53, 96^3 7.5 / 7.5; COMPLEX 64^3 4.37 / 4.40, 96^3 9.2 / 9.2.
-bool resident_plan(int level, int N, int sms, ResidentPlan* out) {
-  if (level != LFM_REAL && level != LFM_COMPLEX) return false;
-  if (N < 8 || N > 128) return false;
+//
+// plans[c]: the cheapest cut of at most c blocks (c = 0: none), for c up to 148.
+static const std::vector<ResidentPlan>& resident_plans(int level, int N) {
+  static std::mutex mu;
+  static std::map<std::pair<int, int>, std::vector<ResidentPlan>> tables;  // at most 2 x 121
+  std::lock_guard<std::mutex> lk(mu);
+  std::vector<ResidentPlan>& plans = tables[{level, N}];
+  if (!plans.empty()) return plans;
+  plans.resize(kMaxBlocks + 1);
   const bool cx = level == LFM_COMPLEX;
   const int ns = cx ? 3 : 2, V = kCells, np = (ns * V + 2) / 3;
   const int N4 = (N + 3) / 4 * 4, RS = N4 + 4;
   const int field = cx ? kFieldFloats<LFM_COMPLEX> : kFieldFloats<LFM_REAL>;
   const int groups = (N + V - 1) / V;
-  static std::mutex mu;
-  static std::map<std::array<int, 3>, ResidentPlan> plans;  // at most 2 x 121 per SM count
-  std::lock_guard<std::mutex> lk(mu);
-  const std::array<int, 3> key{level, N, sms};
-  auto it = plans.find(key);
-  if (it != plans.end()) {
-    *out = it->second;
-    return out->nbi > 0;
-  }
-  ResidentPlan best;
-  double best_t = 1e300;
-  for (int nbi = 1; nbi <= std::min(N, sms); ++nbi) {
-    for (int nbj = 1; nbj <= std::min(N, sms / nbi); ++nbj) {
+  for (int nbi = 1; nbi <= std::min(N, kMaxBlocks); ++nbi) {
+    for (int nbj = 1; nbj <= std::min(N, kMaxBlocks / nbi); ++nbj) {
       const int NI = (N + nbi - 1) / nbi, NJ = (N + nbj - 1) / nbj;
       const int lanes = NJ * groups;
       if (lanes > kMaxThreads) continue;
@@ -656,20 +692,105 @@ bool resident_plan(int level, int N, int sms, ResidentPlan* out) {
       if (smem > kSmemBytes) continue;
       for (int segs = 1; segs <= std::min(NI, kMaxThreads / lanes); ++segs) {
         const int warps = (segs * lanes + 31) / 32, planes = (NI + segs - 1) / segs;
-        const double issue = cx ? (warps > 12 ? 620.0 : 480.0) : 330.0;
+        if (32 * warps > (cx ? kThreadsComplex : kMaxThreads)) break;
+        const double issue = cx ? 480.0 : 330.0;
         const double t = (planes + 0.5) * std::max((warps + 3) / 4 * issue, cx ? 1200.0 : 900.0) +
                          0.7 * halo * groups * np + 2300.0;
-        if (t < best_t) {
-          best_t = t;
+        ResidentPlan& best = plans[nbi * nbj];
+        if (best.nbi == 0 || t < best.cycles)
           best = ResidentPlan{nbi, nbj, NI, NJ, V, segs, warps * 32, RS, smem,
-                              4 + 8LL * nbi * nbj * 2 * (NI + NJ) * np * groups};
-        }
+                              4 + 8LL * nbi * nbj * 2 * (NI + NJ) * np * groups, t};
       }
     }
   }
-  plans[key] = best;
-  *out = best;
-  return best.nbi > 0;
+  for (int c = 1; c <= kMaxBlocks; ++c)
+    if (plans[c].nbi == 0 || (plans[c - 1].nbi && plans[c - 1].cycles <= plans[c].cycles))
+      plans[c] = plans[c - 1];
+  return plans;
+}
+
+bool resident_plan(int level, int N, int sms, ResidentPlan* out) {
+  if ((level != LFM_REAL && level != LFM_COMPLEX) || N < 8 || N > 128 || sms < 1) return false;
+  *out = resident_plans(level, N)[std::min(sms, kMaxBlocks)];
+  return out->nbi > 0;
+}
+
+// Packs the lattices of one level into waves: with a step time T in mind each takes
+// the fewest blocks that make a step in T (or as fast as it can), the largest go
+// first into the first wave with room, and what a wave has left speeds its slowest
+// lattice up.  The T of the smallest total is taken.
+static double pack_level(const int* N, const std::vector<int>& idx, int level, int sms,
+                         std::vector<ResidentWavePlan>* out) {
+  double best_total = 1e300;
+  std::vector<ResidentWavePlan> best;
+  for (double T = 4000.0; T < 60000.0; T *= 1.12) {
+    std::vector<std::pair<int, int>> need;  // blocks, lattice
+    for (int l : idx) {
+      const std::vector<ResidentPlan>& p = resident_plans(level, N[l]);
+      int c = sms;
+      while (c > 1 && p[c - 1].nbi && p[c - 1].cycles <= std::max(T, p[sms].cycles)) --c;
+      need.push_back({p[c].nbi * p[c].nbj, l});
+    }
+    std::stable_sort(need.begin(), need.end(),
+                     [](const auto& a, const auto& b) { return a.first > b.first; });
+    std::vector<ResidentWavePlan> waves;
+    for (const auto& n : need) {
+      const int c = n.first, l = n.second;
+      auto w = std::find_if(waves.begin(), waves.end(), [&](const ResidentWavePlan& v) {
+        return v.blocks + c <= sms && (int)v.lattices.size() < kWaveLattices;
+      });
+      if (w == waves.end()) w = waves.insert(waves.end(), ResidentWavePlan{level, 0, {}, {}});
+      w->blocks += c;
+      w->lattices.push_back(l);
+      w->plans.push_back(resident_plans(level, N[l])[c]);
+    }
+    double total = 0.0;
+    for (ResidentWavePlan& w : waves) {
+      while (true) {
+        size_t slow = 0;
+        for (size_t k = 1; k < w.plans.size(); ++k)
+          if (w.plans[k].cycles > w.plans[slow].cycles) slow = k;
+        const ResidentPlan& now = w.plans[slow];
+        const int used = now.nbi * now.nbj;
+        const ResidentPlan& more =
+            resident_plans(level, N[w.lattices[slow]])[used + sms - w.blocks];
+        if (more.cycles >= now.cycles) {
+          total += now.cycles;
+          break;
+        }
+        w.blocks += more.nbi * more.nbj - used;
+        w.plans[slow] = more;
+      }
+    }
+    if (total < best_total) {
+      best_total = total;
+      best.swap(waves);
+    }
+  }
+  out->insert(out->end(), best.begin(), best.end());
+  return best_total;
+}
+
+bool resident_waves(const int* level, const int* N, int count, int sms,
+                    std::vector<ResidentWavePlan>* waves, double* cycles) {
+  sms = std::min(sms, kMaxBlocks);
+  *cycles = 0.0;
+  waves->clear();
+  for (int lv : {LFM_REAL, LFM_COMPLEX}) {
+    std::vector<int> idx;
+    for (int l = 0; l < count; ++l) {
+      ResidentPlan p;
+      if (!resident_plan(level[l], N[l], sms, &p) || N[l] % 2) return false;
+      if (level[l] == lv) idx.push_back(l);
+    }
+    if (!idx.empty()) *cycles += pack_level(N, idx, lv, sms, waves);
+  }
+  return true;
+}
+
+cudaError_t launch_resident_wave(const ResidentArgs* a, int count, cudaStream_t stream) {
+  return a[0].level == LFM_REAL ? launch_wave<LFM_REAL>(a, count, stream)
+                                : launch_wave<LFM_COMPLEX>(a, count, stream);
 }
 
 cudaError_t launch_resident(const ResidentArgs& a, cudaStream_t stream) {

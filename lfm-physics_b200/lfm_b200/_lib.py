@@ -106,6 +106,7 @@ _SIGNATURES = {
                                                     POINTER(c_void_p), c_int] + [_D] * 6 + [_P],
     "lfm_batch_create": [POINTER(LatticeDesc), c_int, POINTER(BatchTuning), POINTER(c_void_p)],
     "lfm_batch_step": [_P, c_int, c_int, _P],
+    "lfm_batch_run": [_P, c_int, c_int, c_int, _P],
     "lfm_batch_info": [_P] + [POINTER(c_int)] * 4,
     "lfm_batch_destroy": [_P],
     "lfm_batch_plan": [POINTER(LatticeDesc), c_int, POINTER(BatchTuning), c_int, POINTER(c_int32),

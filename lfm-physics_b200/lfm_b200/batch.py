@@ -109,6 +109,8 @@ class BatchedLattices:
         self._damp = False
         self._graphs: dict = {}
         self.tune_report = None
+        # a tuning of the tile kernel given by the caller asks for that kernel
+        self._on_chip = tuning is None or tuning == "auto"
         if tuning == "auto":
             from .autotune import tune_batch
 
@@ -162,6 +164,20 @@ class BatchedLattices:
         self._cur = 1 - self._cur
         self._damp = True
 
+    run_block = 4096
+    """Most steps per on-chip launch (bounds a launch's length)."""
+
+    def _run_on_chip(self, steps: int) -> bool:
+        """`steps` steps with the lattices held on chip, wave after wave (lfm_batch_run);
+        False if one of them does not fit or a step path is forced."""
+        if not _lib.run_steps("lfm_batch_run", self._handle, steps, self._cur,
+                              1 if self._damp else 0, _stream_handle(self.device)):
+            return False
+        self._cur = (self._cur + steps) % 2
+        self._damp = True
+        self.step += steps
+        return True
+
     def _block_graph(self, steps: int):
         import torch
 
@@ -195,6 +211,10 @@ class BatchedLattices:
             for _ in range(steps):
                 self._step()
             self.step += steps
+            return
+        while self._on_chip and steps >= 2 and self._run_on_chip(min(steps, self.run_block)):
+            steps -= min(steps, self.run_block)
+        if not steps:
             return
         if not self._damp:
             self._step()  # the first step after a host write does not damp prev

@@ -151,3 +151,55 @@ def test_two_lattices_on_two_streams(be):
         b.evolve(200)
         _same(a, b)
         a.synchronize()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes", [[(8, REAL), (108, REAL), (96, COMPLEX), (12, COMPLEX)],
+                                   [(32, REAL)] * 40 + [(32, COMPLEX)] * 35,
+                                   [(96, REAL), (64, COMPLEX), (80, COMPLEX), (48, REAL)] * 2])
+def test_batch_waves_equal_single_steps(be, sizes):
+    """Smallest and largest lattices, more than a wave's lattices, mixed waves: each lattice
+    comes out as the one-step batch kernel gives it, at odd and even step counts."""
+    import torch
+
+    from lfm_b200.batch import BatchedLattices
+
+    cfgs = [(gravity_em if lv else gravity_only)(n, kappa=(1 + i % 3) / 63.0)
+            for i, (n, lv) in enumerate(sizes)]
+    a, b = BatchedLattices(cfgs, backend=be), BatchedLattices(cfgs, backend=be)
+    b._on_chip = False
+    rng = np.random.default_rng(len(sizes))
+    for i, (n, lv) in enumerate(sizes):
+        f = [(0.5 * rng.standard_normal((n, n, n))).astype(np.float32) for _ in range(3)]
+        for e in (a, b):
+            e.set_psi_real(i, f[0])
+            e.set_psi_real_prev(i, f[2])
+            if lv:
+                e.set_psi_imag(i, f[1])
+            e.set_chi(i, (19.0 + 1e-2 * f[2]).astype(np.float32))
+    a.run_block = 6
+    for steps in (4, 5, 13):
+        a.evolve(steps)
+        b.evolve(steps)
+        assert (a._cur, a.step) == (b._cur, b.step)
+        for i in range(len(sizes)):
+            sa, sb = a.device_state(i), b.device_state(i)
+            for k in sa:
+                assert torch.equal(sa[k].view(torch.int32), sb[k].view(torch.int32)), (i, k)
+    a.get_chi(0)  # raises if a wait gave up
+
+
+@pytest.mark.gpu
+def test_batch_keeps_single_steps_where_it_must(be):
+    from lfm_b200.batch import BatchedLattices
+
+    big = BatchedLattices([gravity_only(112), gravity_only(32)], backend=be)
+    assert not big._run_on_chip(4)  # 112^3 does not fit
+    assert not BatchedLattices([gravity_only(32)], backend=be, tuning={"threads": 256})._on_chip
+    small = BatchedLattices([gravity_only(32)], backend=be)
+    assert not small._run_on_chip(1)
+    _lib.set_step_path(_lib.PATH_DIRECT)
+    try:
+        assert not small._run_on_chip(4)
+    finally:
+        _lib.set_step_path(_lib.PATH_AUTO)
