@@ -368,6 +368,18 @@ int lfm_adjoint_step_f32(int level, const float* psi_r, const float* psi_i, cons
                          double kappa, double lambda_self, double chi0, double e0_sq,
                          double epsilon_w, void* stream);
 
+/* The same step in a chain of them: with chain bit 0 the adjoints of psi_r, psi_i and chi
+ * come in as a step with bit 1 left them (multiplied by 1 - mask; chi's zero where chi
+ * was clamped; chi_next is not read), with bit 1 they go out that way for the step
+ * before.  A chain that starts without bit 0 and ends without bit 1 gives the same bits
+ * as the single steps. */
+int lfm_adjoint_chain_f32(int level, const float* psi_r, const float* psi_i, const float* chi,
+                          const float* chi_next, const float* mask_table,
+                          const lfm_mask_lut* lut, const float* const* g_out,
+                          float* const* g_in, int chain, int N, double dt2, double kappa,
+                          double lambda_self, double chi0, double e0_sq, double epsilon_w,
+                          void* stream);
+
 /* ------------------------------------------------------------------------
  * Batches of independent lattices (the runs lfm/sweep.py:14-157 makes one
  * Simulation at a time), stepped together: one launch per step, persistent

@@ -939,6 +939,16 @@ int lfm_adjoint_step_f32(int level, const float* psi_r, const float* psi_i, cons
                          const float* const* g_out, float* const* g_in, int N, double dt2,
                          double kappa, double lambda_self, double chi0, double e0_sq,
                          double epsilon_w, void* stream) {
+  return lfm_adjoint_chain_f32(level, psi_r, psi_i, chi, chi_next, mask_table, lut, g_out, g_in,
+                               0, N, dt2, kappa, lambda_self, chi0, e0_sq, epsilon_w, stream);
+}
+
+int lfm_adjoint_chain_f32(int level, const float* psi_r, const float* psi_i, const float* chi,
+                          const float* chi_next, const float* mask_table, const lfm_mask_lut* lut,
+                          const float* const* g_out, float* const* g_in, int chain, int N,
+                          double dt2, double kappa, double lambda_self, double chi0, double e0_sq,
+                          double epsilon_w, void* stream) {
+  if (chain < 0 || chain > 3) return fail(LFM_ERR_INVALID_ARG, "chain %d not in [0, 3]", chain);
   if (level != LFM_REAL && level != LFM_COMPLEX)
     return fail(LFM_ERR_UNSUPPORTED, "adjoint step: level %d (REAL and COMPLEX only)", level);
   int rc = check_n(N);
@@ -967,7 +977,7 @@ int lfm_adjoint_step_f32(int level, const float* psi_r, const float* psi_i, cons
   const lfm::StepConsts c =
       lfm::make_step_consts(dt2, kappa, lambda_self, chi0, e0_sq, epsilon_w, 0, 0, 0, 0);
   cudaError_t e = lfm::launch_adjoint_step(level, N, psi_r, psi_i, chi, chi_next,
-                                           device_lut(mask_table, lut), g_out, g_in, c,
+                                           device_lut(mask_table, lut), g_out, g_in, c, chain,
                                            static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "adjoint step launch");
   return LFM_OK;

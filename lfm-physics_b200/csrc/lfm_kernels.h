@@ -94,9 +94,11 @@ cudaError_t launch_poisson_finish(const double* dchi, float* chi, int N, float c
 
 // Adjoint step (adjoint.cu).  g_out / g_in: adjoints of (psi_r, psi_r_prev,
 // psi_i, psi_i_prev, chi, chi_prev) after / before the step.
+// chain: bit 0, the incoming psi_r, psi_i, chi adjoints are those of a chained step
+// (already multiplied); bit 1, the outgoing ones are left so for the next.
 cudaError_t launch_adjoint_step(int level, int N, const float* pr, const float* pi,
                                 const float* chi, const float* chi_next, const MaskLut& lut,
                                 const float* const g_out[6], float* const g_in[6],
-                                const StepConsts& c, cudaStream_t stream);
+                                const StepConsts& c, int chain, cudaStream_t stream);
 
 }  // namespace lfm

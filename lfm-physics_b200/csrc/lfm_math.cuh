@@ -222,11 +222,12 @@ __device__ __forceinline__ T current_axis(T pr, T pi, T pr_p, T pr_m, T pi_p, T 
   return fsub(fmul(pr, fsub(pi_p, pi_m)), fmul(pi, fsub(pr_p, pr_m)));
 }
 
-// lap19 of two cells at once.  The neighbours in i and j sit at the same
-// vector position as the cells, so those sums run packed; the k-neighbours
-// (k-1, k+1) are the next cell over, so those adds run per lane.  The order
-// of every cell's additions is the one lap19 uses.
-__device__ __forceinline__ F2 lap19_pair(const S19& a, const S19& b) {
+// lap19's face and edge sums (and lap19) of two cells at once.  The neighbours
+// in i and j sit at the same vector position as the cells, so those sums run
+// packed; the k-neighbours (k-1, k+1) are the next cell over, so those adds
+// run per lane.  The order of every cell's additions is the one lap19 uses.
+__device__ __forceinline__ void sums19_pair(const S19& a, const S19& b, F2& face_sum,
+                                            F2& edge_sum) {
   F2 faces = fadd(pk(a.im, b.im), pk(a.ip, b.ip));
   faces = fadd(faces, pk(a.jm, b.jm));
   faces = fadd(faces, pk(a.jp, b.jp));
@@ -245,9 +246,16 @@ __device__ __forceinline__ F2 lap19_pair(const S19& a, const S19& b) {
   ea = fadd(ea, a.jmkp); eb = fadd(eb, b.jmkp);
   ea = fadd(ea, a.jpkm); eb = fadd(eb, b.jpkm);
   ea = fadd(ea, a.jpkp); eb = fadd(eb, b.jpkp);
+  face_sum = pk(fa, fb);
+  edge_sum = pk(ea, eb);
+}
+
+__device__ __forceinline__ F2 lap19_pair(const S19& a, const S19& b) {
+  F2 faces, edges;
+  sums19_pair(a, b, faces, edges);
   const float face_w = (float)(1.0 / 3.0);
   const float edge_w = (float)(1.0 / 6.0);
-  return fadd(fadd(fmul(cst<F2>(face_w), pk(fa, fb)), fmul(cst<F2>(edge_w), pk(ea, eb))),
+  return fadd(fadd(fmul(cst<F2>(face_w), faces), fmul(cst<F2>(edge_w), edges)),
               fmul(cst<F2>(-4.0f), pk(a.c, b.c)));
 }
 

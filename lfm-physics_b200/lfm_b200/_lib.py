@@ -104,6 +104,9 @@ _SIGNATURES = {
     + [_P],
     "lfm_adjoint_step_f32": [c_int] + [_P] * 5 + [POINTER(MaskLut), POINTER(c_void_p),
                                                     POINTER(c_void_p), c_int] + [_D] * 6 + [_P],
+    "lfm_adjoint_chain_f32": [c_int] + [_P] * 5 + [POINTER(MaskLut), POINTER(c_void_p),
+                                                     POINTER(c_void_p), c_int, c_int]
+    + [_D] * 6 + [_P],
     "lfm_batch_create": [POINTER(LatticeDesc), c_int, POINTER(BatchTuning), POINTER(c_void_p)],
     "lfm_batch_step": [_P, c_int, c_int, _P],
     "lfm_batch_run": [_P, c_int, c_int, c_int, _P],

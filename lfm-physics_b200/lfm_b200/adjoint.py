@@ -161,15 +161,16 @@ class _Lattice:
                   ctypes.byref(self.desc), int(damp), self.N, *self.common,
                   float(self.config.epsilon_w), _stream_handle(self.device))
 
-    def adjoint_step(self, st, nx, g_out, g_in) -> None:
-        """The gradient back through the step from state buffer st to nx."""
+    def adjoint_step(self, st, nx, g_out, g_in, chain: int = 0) -> None:
+        """The gradient back through the step from state buffer st to nx (chain: as
+        lfm_adjoint_chain_f32)."""
         ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
         go = (ctypes.c_void_p * 6)(*[ptr(t) for t in g_out])
         gi = (ctypes.c_void_p * 6)(*[ptr(t) for t in g_in])
-        _lib.call("lfm_adjoint_step_f32", int(self.level), st[0].data_ptr(), ptr(st[1]),
+        _lib.call("lfm_adjoint_chain_f32", int(self.level), st[0].data_ptr(), ptr(st[1]),
                   self.chi32(st, 0).data_ptr(), self.chi32(nx, 1).data_ptr(),
                   self.table.data_ptr(),
-                  ctypes.byref(self.desc), go, gi, self.N, *self.common,
+                  ctypes.byref(self.desc), go, gi, int(chain), self.N, *self.common,
                   float(self.config.epsilon_w), _stream_handle(self.device))
 
 
@@ -339,8 +340,11 @@ class _Plan:
                     lat.advance(states[u], p0 if u == 0 else states[u - 1], states[u + 1],
                                 self.meta[si] if u == 0 else True)
             for t in range(e0 - 1, s0 - 1, -1):
+                # every step but the run's last (the first walked) takes its adjoints as
+                # the step before in the walk left them, all but its first leave them so
+                chain = (1 if t < steps - 1 else 0) | (2 if t > 0 else 0)
                 lat.adjoint_step(states[t - s0], states[t - s0 + 1], self.g[cur],
-                                 self.g[1 - cur])
+                                 self.g[1 - cur], chain)
                 cur = 1 - cur
         return cur
 
