@@ -374,61 +374,41 @@ __device__ __forceinline__ bool receive(float* sm, const Block& B, const Cells& 
   return true;
 }
 
-// Copies rows listed in `rows` (global row numbers, -1 = none) of one array into
-// shared memory, row r at dst + 4 + r * RS, with the copies beyond its ends.  A warp
-// takes a row, eight rows' loads in flight (one at a time, filling a block of COMPLEX
-// 96^3 took 50 us).
+template <int BYTES>
+__device__ __forceinline__ void copy_async(float* dst, const float* src) {
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  if constexpr (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
+}
+
+// Starts the copies of rows listed in `rows` (global row numbers, -1 = none) of one
+// array into shared memory, row r at dst + 4 + r * RS; a warp takes a row.  All of a
+// block's copies are in flight at once (a row's loads at a time, then its stores,
+// filled a block of COMPLEX 96^3 in 50 us).
 __device__ __forceinline__ void copy_rows(const float* src, float* dst, const int* rows,
                                           int count, const Block& B, int warp, int nwarps,
                                           int lane) {
-  constexpr int U = 8;
-  if ((B.N & 3) == 0) {
-    const int n4 = B.N >> 2;  // at most 32
-    for (int r = warp; r < count; r += U * nwarps) {
-      float4 t[U];
-      bool have[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int q = r + u * nwarps;
-        have[u] = q < count && lane < n4 && rows[q] >= 0;
-        if (have[u]) t[u] = *(reinterpret_cast<const float4*>(src + rows[q] * B.N) + lane);
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if (!have[u]) continue;
-        float* d = dst + 4 + (r + u * nwarps) * B.RS;
-        reinterpret_cast<float4*>(d)[lane] = t[u];
-        if (lane == 0) d[B.N] = t[u].x;
-        if (lane == n4 - 1) d[-1] = t[u].w;
-      }
+  for (int r = warp; r < count; r += nwarps) {
+    if (rows[r] < 0) continue;
+    const float* s = src + rows[r] * B.N;
+    float* d = dst + 4 + r * B.RS;
+    if ((B.N & 3) == 0) {  // at most 32 groups of four
+      if (4 * lane < B.N) copy_async<16>(d + 4 * lane, s + 4 * lane);
+    } else {
+      for (int k = lane; k < B.N; k += 32) copy_async<4>(d + k, s + k);
     }
-  } else {
-    for (int r = warp; r < count; r += U / 4 * nwarps) {
-      float t[U / 4][4];
-#pragma unroll
-      for (int u = 0; u < U / 4; ++u) {
-        const int q = r + u * nwarps;
-        if (q >= count || rows[q] < 0) continue;
-        const float* s = src + rows[q] * B.N;
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (lane + 32 * k < B.N) t[u][k] = s[lane + 32 * k];
-      }
-#pragma unroll
-      for (int u = 0; u < U / 4; ++u) {
-        const int q = r + u * nwarps;
-        if (q >= count || rows[q] < 0) continue;
-        float* d = dst + 4 + q * B.RS;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int c = lane + 32 * k;
-          if (c >= B.N) continue;
-          d[c] = t[u][k];
-          if (c == 0) d[B.N] = t[u][k];
-          if (c == B.N - 1) d[-1] = t[u][k];
-        }
-      }
-    }
+  }
+}
+
+// The copies beyond the ends of rows [0, count) at dst, once the rows are there.
+__device__ __forceinline__ void copy_ends(float* dst, int count, const Block& B) {
+  for (int r = threadIdx.x; r < count; r += blockDim.x) {
+    float* d = dst + 4 + r * B.RS;
+    const float first = d[0], last = d[B.N - 1];
+    d[B.N] = first;
+    d[-1] = last;
   }
 }
 
@@ -518,13 +498,19 @@ __global__ void __launch_bounds__(THREADS, 1)
     copy_rows(A.prev[f], d + B.SLOT, own_row, L.NI * L.NJ, B, warp, nwarps, lane);
     copy_rows(A.cur[f], d + 2 * B.SLOT, halo_row, HR, B, warp, nwarps, lane);
   }
-#pragma unroll 4
-  for (int x = tid; x < L.NI * L.NJ * B.N4; x += blockDim.x) {
-    const int r = x / B.N4, k = x - r * B.N4;
-    mask_rows[x] = mask_from_q_flat(A.lut, qterm(B.i0 + r / L.NJ, A.N) +
-                                               qterm(B.j0 + r % L.NJ, A.N) +
-                                               qterm(k < A.N ? k : 0, A.N));
+  for (int r = warp; r < L.NI * L.NJ; r += nwarps) {
+    const int q = qterm(B.i0 + r / L.NJ, A.N) + qterm(B.j0 + r % L.NJ, A.N);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int k = lane + 32 * u;
+      if (k < B.N4)
+        mask_rows[r * B.N4 + k] = mask_from_q_flat(A.lut, q + qterm(k < A.N ? k : 0, A.N));
+    }
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+#pragma unroll
+  for (int f = 0; f < NS; ++f) copy_ends(sm + f * FS, 2 * L.NI * L.NJ + HR, B);
 
   Cells T;
   T.groups = groups;
@@ -553,6 +539,9 @@ __global__ void __launch_bounds__(THREADS, 1)
       p = A.stores[s * NS + f];
     s_dst.p[tid / NS][f] = p;
   };
+  // whether step s may store: the destinations are looked at only then (the reads
+  // cost REAL 32^3 7 % of its step)
+  const auto stores = [&](int s) { return A.stores != nullptr || s >= A.steps - 2; };
   set_destination(0);
   __syncthreads();
 
@@ -562,7 +551,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     S.cur = s & 1;
     S.to_prev = (1 - 2 * S.cur) * B.SLOT;
     S.damp = s > 0 || A.damp_first;
-    S.store = s_dst.p[0][0] != nullptr || s_dst.p[1][0] != nullptr;
+    S.store = stores(s);
     S.t = base + (uint32_t)(s + 1);
     ulonglong2* packets = A.packets + (S.t & 1u) * buffer;
     S.out = packets + (int64_t)b * OR * NP * groups;
@@ -590,7 +579,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       s_abort = 1;
       atomicOr(A.status, LFM_ERR_DEVICE_TIMEOUT);
     }
-    set_destination(s + 1);  // behind receive()'s barrier: step s has stored
+    if (stores(s + 1)) set_destination(s + 1);  // behind receive()'s barrier: step s has stored
     __syncthreads();
     if (s_abort) break;
   }
