@@ -119,14 +119,13 @@ int run_step(lfm::StepArgs& a, cudaStream_t stream) {
   const int path = g_path.load();
   cudaError_t e = cudaErrorNotSupported;
   if (path != 1) {
-    e = lfm::launch_tma_step(a, stream);
+    e = lfm::launch_tma_step(a, path == 2, stream);
     if (e != cudaSuccess && e != cudaErrorNotSupported) return cuda_fail(e, "fused step launch");
     if (e == cudaErrorNotSupported && path == 2)
       return fail(LFM_ERR_UNSUPPORTED, "no fused-kernel configuration for N=%d level=%d", a.N,
                   a.level);
   }
   if (e == cudaErrorNotSupported && path == 0) {
-    // measured against the direct kernel at every size it takes (step_march.cu)
     e = lfm::launch_march_step(a, stream);
     if (e != cudaSuccess && e != cudaErrorNotSupported) return cuda_fail(e, "march step launch");
   }

@@ -57,8 +57,9 @@ cudaError_t launch_direct_step(const StepArgs& a, cudaStream_t stream);
 cudaError_t launch_march_step(const StepArgs& a, cudaStream_t stream);
 
 // Fused 2.5D kernel (N % 4 == 0).  Returns cudaErrorNotSupported when the
-// size has no tile configuration, so the caller can take the direct path.
-cudaError_t launch_tma_step(const StepArgs& a, cudaStream_t stream);
+// size has no tile configuration, or (unless any_tile) none that pays beside the
+// marching kernel, so the caller can take another path.
+cudaError_t launch_tma_step(const StepArgs& a, bool any_tile, cudaStream_t stream);
 
 // A bounded wait that must give up (failure-detection test, step_tma.cu).
 cudaError_t launch_wait_selftest(int* status, uint64_t limit_ns, cudaStream_t stream);

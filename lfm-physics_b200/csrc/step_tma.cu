@@ -1569,8 +1569,27 @@ bool try_color(TmaParams& P, const Choice& ch, cudaStream_t stream, cudaError_t*
   return false;
 }
 
+// Whether a run-time tile is still the faster kernel where the marching kernel of
+// step_march.cu runs too.  With its strides in registers the ring's march is slower
+// than that kernel's loads through L1 at every COMPLEX size (us a step, tile against
+// march: 104^3 29.3 / 19.9, 160^3 82.6 / 66.6, 288^3 570 / 336, 384^3 962 / 759), for
+// split chi (REAL 96^3 30.5 / 13.6, 160^3 93.7 / 55.8, COMPLEX 128^3 46.1 / 39.2), the
+// compensated step (REAL 128^3 25.9 / 22.7) and the protocol's streamed mask (COMPLEX
+// 96^3 25.2 / 21.8, REAL 128^3 25.8 / 23.1).  The plain REAL step keeps its tile where
+// it fills a CTA of 384 threads or more on a lattice of 192^3 or more (192^3 61.5 /
+// 66.2, 224^3 92.4 / 96.7, 240^3 113 / 125, 384^3 443 / 450); smaller ones lose as well
+// (112^3 19.9 / 15.9, 144^3 43.5 / 26.2, 176^3 65.8 / 48.5, 288^3 253 / 194).
+template <int LEVEL, bool QUEUE, int MODE>
+bool run_time_tile_pays(const TmaParams& P, const Choice& ch) {
+  if (!QUEUE) return true;  // COLOR has no marching kernel
+  return LEVEL == LFM_REAL && MODE == kPlain && P.pf_mask < 0 && P.N >= 192 && ch.threads >= 384;
+}
+
+// any_tile: the caller asks for the fused kernel, whichever is faster.
 template <int LEVEL, int V, bool QUEUE, int MODE = kPlain>
-cudaError_t plan_and_launch(TmaParams& P, const TileConfig* forced, cudaStream_t stream) {
+cudaError_t plan_and_launch(TmaParams& P, const TileConfig* forced, bool any_tile,
+                            cudaStream_t stream) {
+  any_tile = any_tile || forced;
   using Slot = KernelSlot<LEVEL, V, QUEUE, MODE>;
   int regs = 0;
   cudaError_t e = kernel_regs(Slot::fn(), &regs);
@@ -1617,11 +1636,15 @@ cudaError_t plan_and_launch(TmaParams& P, const TileConfig* forced, cudaStream_t
   // tab[1] lands on a 16-byte boundary: stage_floats is a multiple of N, N of 4
   P.tab_off = tab_in_smem ? ch.S * P.stage_floats + 3 : -1;
   TileConfig used{ch.TJ, ch.S, ch.IC, ch.threads, ch.smem, V};
-  tune_record(LEVEL, P.N, used);
   if constexpr (QUEUE) {
     cudaError_t fe = cudaSuccess;
-    if (try_fixed<LEVEL, V, MODE>(P, ch, stream, &fe)) return fe;
+    if (try_fixed<LEVEL, V, MODE>(P, ch, stream, &fe)) {
+      tune_record(LEVEL, P.N, used);
+      return fe;
+    }
   }
+  if (!any_tile && !run_time_tile_pays<LEVEL, QUEUE, MODE>(P, ch)) return cudaErrorNotSupported;
+  tune_record(LEVEL, P.N, used);
   if constexpr (LEVEL == LFM_COLOR && V == 2) {
     cudaError_t ce = cudaSuccess;
     if (try_color(P, ch, stream, &ce)) return ce;
@@ -1655,7 +1678,7 @@ cudaError_t launch_wait_selftest(int* status, uint64_t limit_ns, cudaStream_t st
   return cudaGetLastError();
 }
 
-cudaError_t launch_tma_step(const StepArgs& a, cudaStream_t stream) {
+cudaError_t launch_tma_step(const StepArgs& a, bool any_tile, cudaStream_t stream) {
   const int N = a.N;
   if (N % 4 != 0 || N < 8) return cudaErrorNotSupported;
   TmaParams P{};
@@ -1723,37 +1746,37 @@ cudaError_t launch_tma_step(const StepArgs& a, cudaStream_t stream) {
     // split chi: two cells per lane (three or four stencil fields, like COMPLEX)
     if (N % 2) return cudaErrorNotSupported;
     // (a tuning recorded for the plain step's tile does not apply)
-    return a.level == LFM_REAL ? plan_and_launch<LFM_REAL, 2, true, kSplit>(P, nullptr, stream)
-                               : plan_and_launch<LFM_COMPLEX, 2, true, kSplit>(P, nullptr, stream);
+    return a.level == LFM_REAL ? plan_and_launch<LFM_REAL, 2, true, kSplit>(P, nullptr, any_tile, stream)
+                               : plan_and_launch<LFM_COMPLEX, 2, true, kSplit>(P, nullptr, any_tile, stream);
   }
   if (a.comp) {
     // compensated Delta form: REAL and COMPLEX, register-queue kernel only
     if (a.level == LFM_REAL)
       return (N % 4) ? cudaErrorNotSupported
-                     : plan_and_launch<LFM_REAL, 4, true, kComp>(P, forced, stream);
+                     : plan_and_launch<LFM_REAL, 4, true, kComp>(P, forced, any_tile, stream);
     if (a.level == LFM_COMPLEX)
       return (N % 2) ? cudaErrorNotSupported
-                     : plan_and_launch<LFM_COMPLEX, 2, true, kComp>(P, forced, stream);
+                     : plan_and_launch<LFM_COMPLEX, 2, true, kComp>(P, forced, any_tile, stream);
     return cudaErrorNotSupported;
   }
   if (a.level == LFM_REAL) {
     const int v = (have_forced && forced_cfg.vec) ? forced_cfg.vec : 4;
     if ((v != 2 && v != 4) || N % v) return cudaErrorNotSupported;
-    return v == 2 ? plan_and_launch<LFM_REAL, 2, true>(P, forced, stream)
-                  : plan_and_launch<LFM_REAL, 4, true>(P, forced, stream);
+    return v == 2 ? plan_and_launch<LFM_REAL, 2, true>(P, forced, any_tile, stream)
+                  : plan_and_launch<LFM_REAL, 4, true>(P, forced, any_tile, stream);
   }
   if (a.level == LFM_COMPLEX) {
     const int v = (have_forced && forced_cfg.vec) ? forced_cfg.vec : 2;
     if ((v != 2 && v != 4) || N % v) return cudaErrorNotSupported;
-    return v == 4 ? plan_and_launch<LFM_COMPLEX, 4, true>(P, forced, stream)
-                  : plan_and_launch<LFM_COMPLEX, 2, true>(P, forced, stream);
+    return v == 4 ? plan_and_launch<LFM_COMPLEX, 4, true>(P, forced, any_tile, stream)
+                  : plan_and_launch<LFM_COMPLEX, 2, true>(P, forced, any_tile, stream);
   }
   // COLOR: two cells per lane, or one when a tuning asks for it (twice the
   // warps on the same ring, each with half the independent arithmetic)
   const int vc = (have_forced && forced_cfg.vec) ? forced_cfg.vec : 2;
   if (vc != 1 && vc != 2) return cudaErrorNotSupported;
-  return vc == 1 ? plan_and_launch<LFM_COLOR, 1, false>(P, forced, stream)
-                 : plan_and_launch<LFM_COLOR, 2, false>(P, forced, stream);
+  return vc == 1 ? plan_and_launch<LFM_COLOR, 1, false>(P, forced, any_tile, stream)
+                 : plan_and_launch<LFM_COLOR, 2, false>(P, forced, any_tile, stream);
 }
 
 

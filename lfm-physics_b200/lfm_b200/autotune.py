@@ -154,14 +154,18 @@ def lattice_candidates(level: int):
 
 
 def tune_lattice(evolver, candidates=None, steps: int = 20, use_cache: bool = True) -> dict:
-    """Pick the fused kernel's tile for the evolver's (level, N) and pin it (lfm_tune_set)."""
+    """Pick the fused kernel's tile for the evolver's (level, N) and pin it (lfm_tune_set).
+
+    A full search (no candidates given) leaves nothing pinned where the kernel that runs
+    without a tile is the faster one ("untuned_is_faster")."""
     level, N = int(evolver._level), int(evolver.N)
     key = f"{_device_name(evolver.device)}|lattice:{level}:{N}"
     if use_cache and candidates is None:
         hit = _load_cache().get(key)
         if hit is not None:
             b = hit["best"]
-            _lib.tune_set(level, N, b["tj"], b["stages"], b["ic"], b["vec"])
+            if not hit.get("untuned_is_faster"):
+                _lib.tune_set(level, N, b["tj"], b["stages"], b["ic"], b["vec"])
             return hit
     if evolver._mode != "resident":
         raise ValueError("tune_lattice needs an Evolver with buffers='resident'")
@@ -171,6 +175,11 @@ def tune_lattice(evolver, candidates=None, steps: int = 20, use_cache: bool = Tr
     saved_state = (evolver._cur, evolver._damp, evolver.step, evolver._use_buffer_A)
     prev_path = None
     trials = []
+    untuned = None
+    if candidates is None:  # the kernel that runs without a tile (on chip, or marching)
+        _lib.tune_set(level, N, 0, 0)
+        evolver.evolve(4)
+        untuned = _time_ms(evolver.device, evolver.evolve, max(steps, 4))
     _lib.set_step_path(_lib.PATH_FUSED)
     try:
         for cand in candidates or lattice_candidates(level):
@@ -187,15 +196,22 @@ def tune_lattice(evolver, candidates=None, steps: int = 20, use_cache: bool = Tr
         for t, s in zip(slots, saved):
             t.copy_(s)
         evolver._cur, evolver._damp, evolver.step, evolver._use_buffer_A = saved_state
+        evolver._energy_ok = False  # |Psi_a|^2 is a trial step's
         evolver._graphs = {}
     if not trials:
         _lib.tune_set(level, N, 0, 0, 0, 0)
         raise RuntimeError(f"no fused tile fits level {level} N={N}")
     best = min(trials, key=lambda t: t["ms_per_step"])
     b = best["tile"]
-    _lib.tune_set(level, N, b["tj"], b["stages"], b["ic"], b["vec"])
     out = {"best": {k: b[k] for k in ("vec", "tj", "stages", "ic")},
            "ms_per_step": best["ms_per_step"], "trials": trials}
+    if untuned is not None:
+        out["untuned_ms_per_step"] = untuned
+        out["untuned_is_faster"] = untuned <= best["ms_per_step"]
+    if out.get("untuned_is_faster"):
+        _lib.tune_set(level, N, 0, 0)
+    else:
+        _lib.tune_set(level, N, b["tj"], b["stages"], b["ic"], b["vec"])
     if candidates is None:
         _store(key, out)
     return out
