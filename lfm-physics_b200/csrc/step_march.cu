@@ -1,4 +1,5 @@
-// Marching step kernel for lattices the copy engine cannot serve (REAL, COMPLEX).
+// Marching step kernels through L1, for lattices the copy engine cannot serve and
+// those it serves more slowly.
 //
 // The fused kernels of step_tma.cu copy rows in 16-byte units, so they need N % 4
 // == 0 and aligned fields.  Here a thread keeps two cells of a row and marches along
@@ -40,6 +41,18 @@ struct Rows {
   int m, z, p, left, two, right;
   bool whole;  // both cells lie in the row
 };
+
+__device__ __forceinline__ Rows rows_at(int N, int j, int k0) {
+  Rows R;
+  R.z = j * N + k0;
+  R.m = (j == 0 ? N - 1 : j - 1) * N + k0;
+  R.p = (j == N - 1 ? 0 : j + 1) * N + k0;
+  R.whole = k0 + 1 < N;
+  R.left = k0 == 0 ? N - 1 : -1;
+  R.two = R.whole ? 1 : -k0;
+  R.right = k0 + V < N ? V : (k0 + V == N ? -k0 : 0);
+  return R;
+}
 
 // The two cells at p; PAIR: as one 8-byte load (N even, aligned fields).
 template <bool PAIR>
@@ -245,14 +258,7 @@ __global__ void __launch_bounds__(kThreads<LEVEL>, 2)
   const int y = (blockIdx.x % tiles) * kThreads<LEVEL> + threadIdx.x;
   if (y >= N * groups) return;
   const int j = y / groups, k0 = (y - j * groups) * V;
-  Rows R;
-  R.z = j * N + k0;
-  R.m = (j == 0 ? N - 1 : j - 1) * N + k0;
-  R.p = (j == N - 1 ? 0 : j + 1) * N + k0;
-  R.whole = k0 + 1 < N;
-  R.left = k0 == 0 ? N - 1 : -1;
-  R.two = R.whole ? 1 : -k0;
-  R.right = k0 + V < N ? V : (k0 + V == N ? -k0 : 0);
+  const Rows R = rows_at(N, j, k0);
   int32_t qjk[V];
 #pragma unroll
   for (int e = 0; e < V; ++e) qjk[e] = qterm(j, N) + qterm(min(k0 + e, N - 1), N);
@@ -286,6 +292,114 @@ __global__ void __launch_bounds__(kThreads<LEVEL>, 2)
   }
 }
 
+// ---- COLOR ------------------------------------------------------------------
+// Seven stencil fields do not fit into a register queue, so a plane's three planes of
+// rows are loaded for each field in turn; marching along i, a CTA finds two of the
+// three in L1.  Two cells a thread run packed, as in the fused kernel.  Without S_a, us
+// a step, against the direct kernel: 50^3 13.8 -> 10.7, 110^3 97.9 -> 68.3, 150^3 256 ->
+// 178, 210^3 711 -> 458; against the fused kernel's run-time tile: 72^3 33.3 -> 23.3,
+// 144^3 214 -> 156, 160^3 241 -> 211, 192^3 372 -> 346.
+template <bool PAIR>
+__global__ void __launch_bounds__(256, 2)
+    march_color_kernel(const __grid_constant__ StepArgs a, int planes, int tiles) {
+  const int N = a.N, groups = (N + 1) / V, n2 = N * N;
+  const int y = (blockIdx.x % tiles) * 256 + threadIdx.x;
+  if (y >= N * groups) return;
+  const int j = y / groups, k0 = (y - j * groups) * V;
+  const Rows R = rows_at(N, j, k0);
+  const int64_t n3 = (int64_t)n2 * N;
+  const int32_t qj0 = qterm(j, N) + qterm(k0, N), qj1 = qterm(j, N) + qterm(min(k0 + 1, N - 1), N);
+  const int i0 = (int)(blockIdx.x / tiles) * planes, i1 = min(i0 + planes, N);
+  const auto pair = [](const Vec<V>& v) { return pk(v.v[0], v.v[1]); };
+  const auto put = [&](float* p, const F2& t) {
+    const float o[V] = {t.v.x, t.v.y};
+    put2<PAIR>(p, o, R);
+  };
+  for (int i = i0; i < i1; ++i) {
+    const int64_t here = (int64_t)i * n2, x = here + R.z;
+    const int64_t before = (int64_t)(i == 0 ? N - 1 : i - 1) * n2;
+    const int64_t after = (int64_t)(i == N - 1 ? 0 : i + 1) * n2;
+    // the Laplacian, centre and faces of field f at the thread's cells
+    S19 c0, c1;
+    const auto gather = [&](const float* f) {
+      QPlane<V> m, c, p;
+      load_plane<PAIR>(m, f + before, R);
+      load_plane<PAIR>(c, f + here, R);
+      load_sides(c, f + here, R);
+      load_plane<PAIR>(p, f + after, R);
+      c0 = q_s19<V>(m, c, p, 0);
+      c1 = q_s19<V>(m, c, p, 1);
+    };
+    F2 mask;
+    if (a.mask) {
+      mask = pair(own2<PAIR>(a.mask + x, R));
+    } else {
+      const int32_t qi = qterm(i, N);
+      mask = pk(mask_from_q_flat(a.lut, qi + qj0), mask_from_q_flat(a.lut, qi + qj1));
+    }
+    F2 prc[3], pic[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      prc[c] = pair(ldg2<PAIR>(a.pr + c * n3 + x, R));
+      pic[c] = pair(ldg2<PAIR>(a.pi + c * n3 + x, R));
+    }
+    gather(a.chi);
+    const F2 lapX = lap19_pair(c0, c1), chi = pk(c0.c, c1.c);
+    ColorAccT<F2> A;
+    color_begin(A, chi, mask, prc, pic, a.c);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      F2 rp = pair(own2<PAIR>(a.pr_prev + c * n3 + x, R));
+      F2 ip = pair(own2<PAIR>(a.pi_prev + c * n3 + x, R));
+      if (a.damp_prev) {
+        rp = fmul(rp, A.absorb);
+        ip = fmul(ip, A.absorb);
+      }
+      gather(a.pr + c * n3);
+      const F2 lapR = lap19_pair(c0, c1), pr = pk(c0.c, c1.c);
+      const FacesT<F2> fr = pk_faces(faces_of(c0), faces_of(c1));
+      gather(a.pi + c * n3);
+      const ColorCompOutT<F2> o =
+          color_component(A, c, lapR, pr, rp, fr, lap19_pair(c0, c1), pk(c0.c, c1.c), ip,
+                          pk_faces(faces_of(c0), faces_of(c1)), a.c);
+      put(a.pr_out + c * n3 + x, o.pr);
+      put(a.pi_out + c * n3 + x, o.pi);
+      if (a.energy_out)
+        put(a.energy_out + c * n3 + x, fadd(fmul(o.pr, o.pr), fmul(o.pi, o.pi)));
+      if (a.pr_prev_out) put(a.pr_prev_out + c * n3 + x, o.pr_prev);
+      if (a.pi_prev_out) put(a.pi_prev_out + c * n3 + x, o.pi_prev);
+    }
+    F2 sa[3] = {cst<F2>(0.0f), cst<F2>(0.0f), cst<F2>(0.0f)};
+    if (a.sa) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        sa[c] = pair(ldg2<PAIR>(a.sa + c * n3 + x, R));
+        if (a.sa_clip_out)
+          put(a.sa_clip_out + c * n3 + x, pk(fmaxf(sa[c].v.x, 0.0f), fmaxf(sa[c].v.y, 0.0f)));
+      }
+    }
+    const F2 xp = pair(own2<PAIR>(a.chi_prev + x, R));
+    put(a.chi_out + x, color_finish(A, lapX, xp, a.sa != nullptr, sa, a.c));
+    if (a.chi_prev_out) put(a.chi_prev_out + x, chi);
+  }
+}
+
+cudaError_t launch_color(const StepArgs& a, bool pairs, cudaStream_t stream) {
+  const int tiles = (a.N * ((a.N + 1) / V) + 255) / 256;
+  const int64_t work = (int64_t)tiles * a.N;
+  // All CTAs resident at once (2 x 148) while that takes ten planes or fewer (110^3: 68.3
+  // us with nine, 78 with four, 74 with one), four planes beyond (150^3: 178 with four,
+  // 188 with one, 223 with 16).
+  int planes = (int)((work + 295) / 296);
+  if (planes > 10) planes = 4;
+  const unsigned grid = (unsigned)tiles * (unsigned)((a.N + planes - 1) / planes);
+  if (pairs)
+    march_color_kernel<true><<<grid, 256, 0, stream>>>(a, planes, tiles);
+  else
+    march_color_kernel<false><<<grid, 256, 0, stream>>>(a, planes, tiles);
+  return cudaGetLastError();
+}
+
 template <int LEVEL, int MODE>
 cudaError_t launch(const StepArgs& a, bool pairs, cudaStream_t stream) {
   const int threads = kThreads<LEVEL>, range = a.slab ? a.i_hi - a.i_lo : a.N;
@@ -310,7 +424,6 @@ cudaError_t launch(const StepArgs& a, bool pairs, cudaStream_t stream) {
 }  // namespace
 
 cudaError_t launch_march_step(const StepArgs& a, cudaStream_t stream) {
-  if (a.level != LFM_REAL && a.level != LFM_COMPLEX) return cudaErrorNotSupported;
   // Below 32^3 the direct kernel's one-cell threads are done sooner (REAL 30^3: 3.2
   // against 4.2 us a step; COMPLEX 15^3 to 30^3 4.2 either way).
   if (a.N < 32) return cudaErrorNotSupported;
@@ -318,8 +431,14 @@ cudaError_t launch_march_step(const StepArgs& a, cudaStream_t stream) {
   bool pairs = a.N % 2 == 0;
   const void* ptrs[] = {a.pr, a.pi, a.chi, a.pr_prev, a.pi_prev, a.chi_prev, a.pr_out, a.pi_out,
                         a.chi_out, a.pr_prev_out, a.pi_prev_out, a.chi_prev_out, a.mask,
-                        a.chi_lo, a.chi_lo_prev, a.chi_lo_out};
+                        a.chi_lo, a.chi_lo_prev, a.chi_lo_out, a.sa, a.sa_clip_out,
+                        a.energy_out};
   for (const void* p : ptrs) pairs = pairs && (reinterpret_cast<uintptr_t>(p) & 7u) == 0;
+  if (a.level == LFM_COLOR) {
+    // (33^3: direct 6.7, march 8.6; 40^3 7.5, 8.8; 50^3 13.8, 10.7)
+    if (a.N < 45 || a.slab) return cudaErrorNotSupported;
+    return launch_color(a, pairs, stream);
+  }
   if (a.level == LFM_REAL)
     return a.split  ? launch<LFM_REAL, kSplit>(a, pairs, stream)
            : a.comp ? launch<LFM_REAL, kComp>(a, pairs, stream)

@@ -1581,7 +1581,9 @@ bool try_color(TmaParams& P, const Choice& ch, cudaStream_t stream, cudaError_t*
 // (112^3 19.9 / 15.9, 144^3 43.5 / 26.2, 176^3 65.8 / 48.5, 288^3 253 / 194).
 template <int LEVEL, bool QUEUE, int MODE>
 bool run_time_tile_pays(const TmaParams& P, const Choice& ch) {
-  if (!QUEUE) return true;  // COLOR has no marching kernel
+  // COLOR: 72^3 33.3 / 23.3, 144^3 214 / 156, 192^3 372 / 346 with 192 to 288 threads a
+  // CTA; 240^3 573 / 663 with 480
+  if (LEVEL == LFM_COLOR) return ch.threads >= 448;
   return LEVEL == LFM_REAL && MODE == kPlain && P.pf_mask < 0 && P.N >= 192 && ch.threads >= 384;
 }
 
@@ -1643,12 +1645,15 @@ cudaError_t plan_and_launch(TmaParams& P, const TileConfig* forced, bool any_til
       return fe;
     }
   }
-  if (!any_tile && !run_time_tile_pays<LEVEL, QUEUE, MODE>(P, ch)) return cudaErrorNotSupported;
-  tune_record(LEVEL, P.N, used);
   if constexpr (LEVEL == LFM_COLOR && V == 2) {
     cudaError_t ce = cudaSuccess;
-    if (try_color(P, ch, stream, &ce)) return ce;
+    if (try_color(P, ch, stream, &ce)) {
+      tune_record(LEVEL, P.N, used);
+      return ce;
+    }
   }
+  if (!any_tile && !run_time_tile_pays<LEVEL, QUEUE, MODE>(P, ch)) return cudaErrorNotSupported;
+  tune_record(LEVEL, P.N, used);
   return launch_kernel(Slot::fn(), &Slot::granted, &Slot::mu, P, ch, stream);
 }
 

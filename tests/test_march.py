@@ -122,3 +122,32 @@ def test_slabs(be, level, N, ranks):
         _lib.set_step_path(_lib.PATH_AUTO)
     got = np.asarray(gather_local(slabs, "psi_r"))
     assert np.array_equal(got.view(np.uint32), ev.get_psi_real().view(np.uint32))
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("N", [44, 45, 46, 72, 110])
+def test_color_steps(be, N, shift):
+    """COLOR around its smallest marching lattice, odd and even, one and several planes a
+    march, with every coupling (S_a apart, which enters both kernels as the same array)."""
+    import torch
+
+    n = N**3
+    rng = np.random.default_rng(N)
+    psi = [(0.5 * rng.standard_normal(3 * n)).astype(np.float32) for _ in range(4)]
+    ins = psi + _fields(rng, 2, n) + [rng.random(n).astype(np.float32)]
+
+    def dev(a):
+        t = torch.zeros(a.size + shift, dtype=torch.float32, device=be.device)
+        t[shift:] = torch.from_numpy(a).to(be.device)
+        return t[shift:]
+
+    def run():
+        out = [dev(np.zeros_like(a)) for a in ins[:6]]
+        sa = dev(np.zeros(3 * n, np.float32))
+        be.step_color(*[dev(a) for a in ins], *out, N, 4e-4, 1 / 63, 4 / 31, 19.0, 0.01, 0.1,
+                      1 / 189, 2 / 17, kappa_string=1 / 189, kappa_tube=30 / 63,
+                      sa_fields_out=sa)
+        return [be.to_numpy(o).view(np.uint32) for o in out + [sa]]
+
+    for a, b in zip(*_direct(run)):
+        assert np.array_equal(a, b)
