@@ -282,7 +282,7 @@ int filter_table(FftSlot* s, int N, double gamma, double d, cudaStream_t stream,
 // created on first use (outside stream capture: they allocate and upload).
 int split_transform(FftSlot* s, int N, double gamma, double d, cudaStream_t stream,
                     float** table) {
-  if (s->r2c_2d && s->tables.count({gamma, d})) {
+  if (s->twiddles && s->tables.count({gamma, d})) {
     *table = s->tables[{gamma, d}];
     return LFM_OK;
   }
@@ -292,7 +292,7 @@ int split_transform(FftSlot* s, int N, double gamma, double d, cudaStream_t stre
                 N, gamma, d);
   const int nz = N / 2 + 1;
   cudaError_t e = cudaSuccess;
-  if (!s->r2c_2d) {
+  if (!s->r2c_2d && !lfm::plane_transform_supported(N)) {
     int n[2] = {N, N}, inr[2] = {N, N}, inc[2] = {N, nz};
     if (cufftPlanMany(&s->r2c_2d, 2, n, inr, 1, N * N, inc, 1, N * nz, CUFFT_R2C, 3 * N) !=
         CUFFT_SUCCESS)
@@ -300,6 +300,8 @@ int split_transform(FftSlot* s, int N, double gamma, double d, cudaStream_t stre
     if (cufftPlanMany(&s->c2r_2d, 2, n, inc, 1, N * nz, inr, 1, N * N, CUFFT_C2R, 3 * N) !=
         CUFFT_SUCCESS)
       return fail(LFM_ERR_CUFFT, "cufftPlanMany 2-D C2R N=%d", N);
+  }
+  if (!s->twiddles) {
     std::vector<float2> tw(N);
     for (int t = 0; t < N; ++t) {
       const double ang = -2.0 * 3.14159265358979323846 * (double)t / (double)N;
@@ -335,15 +337,26 @@ int helmholtz(lfm_context* ctx, const float* pr, const float* pi, float* sa_raw,
     float* table = nullptr;
     rc = split_transform(s, N, gamma, d, stream, &table);
     if (rc) return rc;
-    if (cufftSetStream(s->r2c_2d, stream) != CUFFT_SUCCESS ||
-        cufftExecR2C(s->r2c_2d, const_cast<float*>(src),
-                     reinterpret_cast<cufftComplex*>(s->spec)) != CUFFT_SUCCESS)
+    const bool planes = lfm::plane_transform_supported(N);
+    if (planes) {
+      e = lfm::launch_plane_transform(false, const_cast<float*>(src), s->spec, s->twiddles, N,
+                                      stream);
+      if (e != cudaSuccess) return cuda_fail(e, "plane transform");
+    } else if (cufftSetStream(s->r2c_2d, stream) != CUFFT_SUCCESS ||
+               cufftExecR2C(s->r2c_2d, const_cast<float*>(src),
+                            reinterpret_cast<cufftComplex*>(s->spec)) != CUFFT_SUCCESS) {
       return fail(LFM_ERR_CUFFT, "cufftExecR2C 2-D N=%d", N);
+    }
     e = lfm::launch_helmholtz_xpass(s->spec, table, s->twiddles, N, stream);
     if (e != cudaSuccess) return cuda_fail(e, "Helmholtz pass along i");
-    if (cufftSetStream(s->c2r_2d, stream) != CUFFT_SUCCESS ||
-        cufftExecC2R(s->c2r_2d, reinterpret_cast<cufftComplex*>(s->spec), dst) != CUFFT_SUCCESS)
+    if (planes) {
+      e = lfm::launch_plane_transform(true, dst, s->spec, s->twiddles, N, stream);
+      if (e != cudaSuccess) return cuda_fail(e, "plane transform");
+    } else if (cufftSetStream(s->c2r_2d, stream) != CUFFT_SUCCESS ||
+               cufftExecC2R(s->c2r_2d, reinterpret_cast<cufftComplex*>(s->spec), dst) !=
+                   CUFFT_SUCCESS) {
       return fail(LFM_ERR_CUFFT, "cufftExecC2R 2-D N=%d", N);
+    }
     if (sa_used) *sa_used = dst;
     return LFM_OK;
   }

@@ -82,6 +82,11 @@ cudaError_t launch_helmholtz_table(float* table, int N, double gamma, double d,
                                    cudaStream_t stream);
 cudaError_t launch_helmholtz_xpass(float2* spec, const float* table, const float2* twiddles,
                                    int N, cudaStream_t stream);
+// The 2-D real transforms over (j, k) of the 3N planes (spectral.cu): which N they
+// serve, and real[3N][N][N] <-> spec[3N][N][N/2+1], unnormalised.
+bool plane_transform_supported(int N);
+cudaError_t launch_plane_transform(bool inverse, float* real, float2* spec, const float2* tw, int N,
+                                   cudaStream_t stream);
 // Uploads the register DFTs' twiddles to the current device's constant memory
 // (once per device, before the first pass along i; synchronous).
 cudaError_t upload_dft_twiddles();

@@ -4,10 +4,10 @@
 //   S_a = IRFFT3[ gamma / (gamma + D |k|^2) * RFFT3(|Psi_a|^2) ]
 // (lfm/core/backends/numpy_backend.py:341-356).  A 3-D transform is three 1-D
 // passes, so the solve is split as
-//   cuFFT 2-D R2C over (j, k) for every plane i and colour
+//   2-D R2C over (j, k) for every plane i and colour (cuFFT, or in one CTA: below)
 //   -> this kernel: forward 1-D FFT along i, times the filter, inverse 1-D FFT
-//   -> cuFFT 2-D C2R over (j, k).
-// The kernel replaces three HBM round trips of the half spectrum (the forward
+//   -> 2-D C2R over (j, k).
+// This kernel replaces three HBM round trips of the half spectrum (the forward
 // pass along i, the filter multiply, the inverse pass along i) by one.
 //
 // Spectrum layout (cuFFT's R2C output): spec[a][x][w], w = y * (N/2+1) + z,
@@ -169,6 +169,195 @@ __global__ void __launch_bounds__(N1* TW) helmholtz_xpass_kernel(float2* __restr
   for (int m = 0; m < N2; ++m) col[(int64_t)(n1 + N1 * m) * W] = v[m];
 }
 
+// ---- 2-D transforms of a plane in one CTA (N = 64, 128) ------------------------
+//
+// cuFFT takes two kernels for the 2-D transform of these planes, each a pass over the
+// data and a launch.  A plane (16 or 64 KB) fits into shared memory, so one CTA does
+// both directions of it: rows two at a time as the real and imaginary part of one
+// complex transform, columns 0 and N/2 of the half spectrum (real for every row) as one
+// column in the same way.  That leaves N/2 complex transforms of length N each way,
+// N1 threads with N2 elements each (the four-step scheme above).  Whole COLOR steps with
+// S_a: 64^3 32.0 -> 28.2 us, 128^3 157 -> 153 (there the stencil takes 91).  A plane of
+// 256^2 (264 KB) does not fit and stays with cuFFT.
+template <int N1, int N2>
+struct PlaneShape {
+  static constexpr int N = N1 * N2, H = N / 2, G = N2 / N1, T = H * N1;
+  // a row transform's exchange rows, padded so that neighbouring transforms start on
+  // other banks; a half-spectrum row, padded for the row-wise accesses
+  static constexpr int LE = N + N1, LS = H + 1;
+  static constexpr int kSmem = (N + (H * LE > N * H ? H * LE : N * H) + N * LS + N) * 8;
+};
+
+// A length-N transform, N1 threads each: v[m] is element n1 + N1 m; at(q): the
+// exchange place of element q of this transform; the thread ends with X[k2 + N2 k1],
+// k2 = n1 + N1 g, in u[g][k1].
+template <int N1, int N2, bool INV, class At>
+__device__ __forceinline__ void fft_split(float2 (&v)[N2], float2 (&u)[N2 / N1][N1], int n1,
+                                          const float2* tw, const At& at) {
+  dft_reg<N2, INV>(v);
+#pragma unroll
+  for (int k2 = 1; k2 < N2; ++k2) {
+    const float2 w = tw[n1 * k2];
+    v[k2] = cmul(v[k2], INV ? conjf2(w) : w);
+  }
+#pragma unroll
+  for (int k2 = 0; k2 < N2; ++k2) *at(k2 * N1 + n1) = v[k2];
+  __syncthreads();
+#pragma unroll
+  for (int g = 0; g < N2 / N1; ++g) {
+#pragma unroll
+    for (int j = 0; j < N1; ++j) u[g][j] = *at((n1 + N1 * g) * N1 + j);
+    dft_reg<N1, INV>(u[g]);
+  }
+}
+
+// spec[plane][y][z] <- the 2-D real transform of real[plane][j][k].
+template <int N1, int N2>
+__global__ void __launch_bounds__(N1* N1* N2 / 2) plane_r2c_kernel(const float* __restrict__ real,
+                                                                   float2* __restrict__ spec,
+                                                                   const float2* __restrict__ twg) {
+  using P = PlaneShape<N1, N2>;
+  constexpr int N = P::N, H = P::H;
+  extern __shared__ float2 smem_p[];
+  float2* tw = smem_p;
+  float2* S = tw + N;          // N x LS half spectrum after the rows
+  float2* C = S + N * P::LS;   // column 0
+  float2* E = C + N;           // exchange
+  const int tid = threadIdx.x;
+  for (int t = tid; t < N; t += P::T) tw[t] = twg[t];
+  const float* in = real + (int64_t)blockIdx.x * N * N;
+  float2* out = spec + (int64_t)blockIdx.x * N * (H + 1);
+  float2 v[N2], u[P::G][N1];
+  {  // rows 2 p and 2 p + 1
+    const int p = tid / N1, n1 = tid % N1;
+    const float *ra = in + 2 * p * N, *rb = ra + N;
+#pragma unroll
+    for (int m = 0; m < N2; ++m) v[m] = make_float2(ra[n1 + N1 * m], rb[n1 + N1 * m]);
+    __syncthreads();  // twiddles
+    fft_split<N1, N2, false>(v, u, n1, tw, [&](int q) { return E + p * P::LE + q; });
+    __syncthreads();
+#pragma unroll
+    for (int g = 0; g < P::G; ++g)
+#pragma unroll
+      for (int k1 = 0; k1 < N1; ++k1) E[p * P::LE + n1 + N1 * g + N2 * k1] = u[g][k1];
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < N2 / 2; ++m) {  // Z[k] = A[k] + i B[k] taken apart
+      const int k = n1 + N1 * m;
+      const float2 z = E[p * P::LE + k], w = E[p * P::LE + (k ? N - k : H)];
+      float2 a, b;
+      if (k == 0) {  // columns 0 and N/2, both real, as one
+        a = make_float2(z.x, w.x);
+        b = make_float2(z.y, w.y);
+      } else {
+        a = make_float2(0.5f * (z.x + w.x), 0.5f * (z.y - w.y));
+        b = make_float2(0.5f * (z.y + w.y), 0.5f * (w.x - z.x));
+      }
+      S[2 * p * P::LS + k] = a;
+      S[(2 * p + 1) * P::LS + k] = b;
+    }
+    __syncthreads();
+  }
+  const int c = tid % H, n1 = tid / H;  // column c
+#pragma unroll
+  for (int m = 0; m < N2; ++m) v[m] = S[(n1 + N1 * m) * P::LS + c];
+  fft_split<N1, N2, false>(v, u, n1, tw, [&](int q) { return E + q * H + c; });
+#pragma unroll
+  for (int g = 0; g < P::G; ++g)
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1) {
+      const int y = n1 + N1 * g + N2 * k1;
+      if (c)
+        out[y * (H + 1) + c] = u[g][k1];
+      else
+        C[y] = u[g][k1];
+    }
+  __syncthreads();
+  for (int y = tid; y < N; y += P::T) {
+    const float2 z = C[y], w = C[y ? N - y : 0];
+    out[y * (H + 1)] = make_float2(0.5f * (z.x + w.x), 0.5f * (z.y - w.y));
+    out[y * (H + 1) + H] = make_float2(0.5f * (z.y + w.y), 0.5f * (w.x - z.x));
+  }
+}
+
+// real[plane][j][k] <- the (unnormalised) inverse of spec[plane][y][z].
+template <int N1, int N2>
+__global__ void __launch_bounds__(N1* N1* N2 / 2) plane_c2r_kernel(const float2* __restrict__ spec,
+                                                                   float* __restrict__ real,
+                                                                   const float2* __restrict__ twg) {
+  using P = PlaneShape<N1, N2>;
+  constexpr int N = P::N, H = P::H;
+  extern __shared__ float2 smem_p[];
+  float2* tw = smem_p;
+  float2* S = tw + N;
+  float2* E = S + N * P::LS + N;
+  const int tid = threadIdx.x;
+  for (int t = tid; t < N; t += P::T) tw[t] = twg[t];
+  const float2* in = spec + (int64_t)blockIdx.x * N * (H + 1);
+  float* out = real + (int64_t)blockIdx.x * N * N;
+  float2 v[N2], u[P::G][N1];
+  {
+    const int c = tid % H, n1 = tid / H;
+#pragma unroll
+    for (int m = 0; m < N2; ++m) {
+      const float2* row = in + (n1 + N1 * m) * (H + 1);
+      v[m] = row[c];
+      if (c == 0) {  // F0 + i F(N/2): both columns' inverses are real
+        const float2 h = row[H];
+        v[m] = make_float2(v[m].x - h.y, v[m].y + h.x);
+      }
+    }
+    __syncthreads();  // twiddles
+    fft_split<N1, N2, true>(v, u, n1, tw, [&](int q) { return E + q * H + c; });
+#pragma unroll
+    for (int g = 0; g < P::G; ++g)
+#pragma unroll
+      for (int k1 = 0; k1 < N1; ++k1) S[(n1 + N1 * g + N2 * k1) * P::LS + c] = u[g][k1];
+    __syncthreads();
+  }
+  const int p = tid / N1, n1 = tid % N1;
+#pragma unroll
+  for (int m = 0; m < N2; ++m) {  // Z[k] = A[k] + i B[k] from the half spectra
+    const int k = n1 + N1 * m, q = k < H ? k : (k == H ? 0 : N - k);
+    const float2 a = S[2 * p * P::LS + q], b = S[(2 * p + 1) * P::LS + q];
+    if (k == 0)
+      v[m] = make_float2(a.x, b.x);
+    else if (k == H)
+      v[m] = make_float2(a.y, b.y);
+    else if (k < H)
+      v[m] = make_float2(a.x - b.y, a.y + b.x);
+    else
+      v[m] = make_float2(a.x + b.y, b.x - a.y);
+  }
+  fft_split<N1, N2, true>(v, u, n1, tw, [&](int q) { return E + p * P::LE + q; });
+#pragma unroll
+  for (int g = 0; g < P::G; ++g)
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1) {
+      const int k = n1 + N1 * g + N2 * k1;
+      out[2 * p * N + k] = u[g][k1].x;
+      out[(2 * p + 1) * N + k] = u[g][k1].y;
+    }
+}
+
+template <int N1, int N2>
+cudaError_t launch_planes(bool inverse, float* real, float2* spec, const float2* tw,
+                          cudaStream_t stream) {
+  using P = PlaneShape<N1, N2>;
+  const void* kernel = inverse ? (const void*)plane_c2r_kernel<N1, N2>
+                               : (const void*)plane_r2c_kernel<N1, N2>;
+  if (P::kSmem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         P::kSmem);
+    if (e != cudaSuccess) return e;
+  }
+  if (inverse)
+    plane_c2r_kernel<N1, N2><<<3 * P::N, P::T, P::kSmem, stream>>>(spec, real, tw);
+  else
+    plane_r2c_kernel<N1, N2><<<3 * P::N, P::T, P::kSmem, stream>>>(real, spec, tw);
+  return cudaGetLastError();
+}
+
 // np.fft.fftfreq(n) * 2*pi for the frequency magnitude f: f * (1.0/n) * 2*pi in
 // float64 (the sign of f does not change k^2).
 __device__ __forceinline__ double wave(int f, int n) {
@@ -225,6 +414,15 @@ cudaError_t upload_dft_twiddles() {
 
 bool helmholtz_xpass_supported(int N) {
   return N == 64 || N == 128 || N == 256 || N == 512 || N == 1024;
+}
+
+bool plane_transform_supported(int N) { return N == 64 || N == 128; }
+
+cudaError_t launch_plane_transform(bool inverse, float* real, float2* spec, const float2* tw, int N,
+                                   cudaStream_t stream) {
+  if (N == 64) return launch_planes<8, 8>(inverse, real, spec, tw, stream);
+  if (N == 128) return launch_planes<8, 16>(inverse, real, spec, tw, stream);
+  return cudaErrorNotSupported;
 }
 
 cudaError_t launch_helmholtz_table(float* table, int N, double gamma, double d,

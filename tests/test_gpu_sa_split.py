@@ -167,3 +167,28 @@ def test_psi_writes_invalidate_the_handed_energy(be):
     for got, want in ((ev.get_psi_real().ravel(), lat.pr), (ev.get_chi().ravel(), lat.chi)):
         err = np.abs(got.astype(np.float64) - want).max() / np.abs(want).max()
         assert err < 1e-5, err
+
+
+@pytest.mark.parametrize("N", [64, 128])
+def test_plane_transforms_against_float64(be, N):
+    """The 2-D transforms that run in one CTA: S_a of noise (every frequency present, rows,
+    columns 0 and N/2 included) within the solve's stated 2e-6 of max S_a of float64."""
+    import torch
+
+    from lfm_b200 import _lib
+
+    rng = np.random.default_rng(N)
+    e = rng.random((3, N, N, N)).astype(np.float32)
+    e[1] *= np.cos(np.pi * np.arange(N))[None, None, :] + 1.0  # column N/2
+    d = torch.from_numpy(e).to(be.device)
+    out = torch.empty_like(d)
+    _lib.call("lfm_helmholtz_sa_from_energy_f32", be.context.handle, d.data_ptr(),
+              out.data_ptr(), N, 0.1, 4.9, torch.cuda.current_stream(be.device).cuda_stream)
+    k = 2 * np.pi * np.fft.fftfreq(N)
+    kz = 2 * np.pi * np.fft.rfftfreq(N)
+    k2 = k[:, None, None] ** 2 + k[None, :, None] ** 2 + kz[None, None, :] ** 2
+    got = out.cpu().numpy()
+    for a in range(3):
+        ref = np.fft.irfftn(0.1 / (0.1 + 4.9 * k2) * np.fft.rfftn(e[a].astype(np.float64)),
+                            s=(N, N, N), axes=(0, 1, 2))
+        assert np.abs(got[a] - ref).max() <= 2e-6 * np.abs(ref).max()
