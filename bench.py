@@ -293,11 +293,22 @@ def run_reference(args):
     return 0
 
 
+def batch_launches(B, steps):
+    """Launches of `steps` steps of a batch, at least: on chip a wave takes up to 32
+    lattices of one level through all steps of a run; else one launch a step."""
+    if not B._on_chip:
+        return steps
+    levels = [int(c.field_level) for c in B.configs]
+    waves = sum(-(-levels.count(lv) // 32) for lv in set(levels))
+    return waves * -(-steps // B.run_block)
+
+
 def run_batched(args, be, dev, rank, barrier, max_over_ranks, peak):
     """Batched sweep: `batch_lattices` lattices (N in {32..96}, REAL/COMPLEX mixed,
-    one packet each) in one persistent launch per step, the whole
-    step loop replayed as one CUDA graph, against the plain loop of
-    single-lattice Evolvers over the same lattices on the same GPU."""
+    one packet each), held on chip wave after wave with all steps of an evolve in
+    one launch a wave, against the plain loop of single-lattice Evolvers over the
+    same lattices on the same GPU.  With --batch-tuning threads,stages,cells: the
+    tile kernel, one persistent launch per step, the step loop as one CUDA graph."""
     import torch
 
     from lfm_b200 import Evolver, _lib
@@ -349,7 +360,7 @@ def run_batched(args, be, dev, rank, barrier, max_over_ranks, peak):
     status = _lib.device_status(clear=True)
     if status:
         raise RuntimeError(f"device status word {status} after the batched steps")
-    info = B.info()
+    info, launches = B.info(), batch_launches(B, steps)
     del B
 
     evs = []
@@ -386,7 +397,7 @@ def run_batched(args, be, dev, rank, barrier, max_over_ranks, peak):
                        "complex": sum(1 for c in cfgs if int(c.field_level) == 1)},
             "plain_loop": {"value": vp, "unit": METRIC, "ms": ms_p,
                            "how": "one Evolver per lattice, evolve(steps) each in turn "
-                                  "(two-step CUDA graphs)"},
+                                  "(on chip, one launch each)"},
             "speedup_vs_plain_loop": ms_p / ms_b,
             "reference_semantics_loop": {
                 "value": cells * steps / (ms_r / 1e3) / 1e9, "unit": METRIC, "ms": ms_r,
@@ -395,7 +406,7 @@ def run_batched(args, be, dev, rank, barrier, max_over_ranks, peak):
             "speedup_vs_reference_semantics_loop": ms_r / ms_b,
             "roofline": {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                          "frac": ach / peak, "bytes_per_cell": "24 REAL / 36 COMPLEX"},
-            "launch": info, "gpu_launches": steps,
+            "launch": info, "gpu_launches": launches,
             "autotune": {"best": tune["best"], "ms_per_step": tune["ms_per_step"],
                          "default_ms_per_step": next(
                              (t["ms_per_step"] for t in tune.get("trials", [])
@@ -520,7 +531,7 @@ def run_adjoint(args, be, dev, barrier, max_over_ranks):
     base = torch.cuda.memory_allocated(dev)
     fwd, bwd, loss, gmax = one(True)
     peak = torch.cuda.max_memory_allocated(dev) - base
-    # the plain forward of the same steps (Evolver, two-step CUDA graphs)
+    # the plain forward of the same steps (Evolver, on chip)
     evp = Evolver(cfg, backend=be)
     evp.set_psi_real(st[0])
     evp.set_psi_imag(st[2])
@@ -863,7 +874,7 @@ def run_slab(args):
 
 def run_sweep_sharded(args):
     """The batched-sweep lattices shared out over the ranks by cost (lfm_b200.sweep.shard);
-    each rank advances its share in one batched launch per step."""
+    each rank advances its share as one batch (on chip, wave after wave)."""
     import torch
     import torch.distributed as dist
 
@@ -907,7 +918,7 @@ def run_sweep_sharded(args):
            "lattices": len(L), "cells": cells, "parallelism": f"lattices sharded x{world}",
            "lattices_this_rank0": len(parts[0]), "l2": "every lattice stepped once per step"}
     line = _common_line(args, cells * steps / (ms / 1e3) / 1e9, ms, world, cfg, "strong",
-                        clock_info, steps)
+                        clock_info, batch_launches(B, steps))
     line["steps"] = steps
     del B
     if world > 1:

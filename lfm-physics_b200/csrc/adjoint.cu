@@ -58,7 +58,7 @@ struct AdjArgs {
 // loads, sums in packed pairs) in kPlanes planes, so that a field's plane is read
 // once for the planes it borders.  The kernel is bound by issue, about 500
 // instructions a COMPLEX cell with one cell a thread and every neighbour loaded
-// where it is used (28.4 us at 96^3); now @@.
+// where it is used (28.4 us at 96^3); now 24.4 us.
 constexpr int TI = 4, TJ = 8, TK = 32;
 constexpr int kPlanes = TI / 2;  // two halves of the CTA share the block's planes
 constexpr int HI = TI + 2, HJ = TJ + 2;

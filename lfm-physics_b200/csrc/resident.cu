@@ -654,8 +654,10 @@ cudaError_t launch_wave(const ResidentArgs* a, int count, cudaStream_t stream) {
 // exchange.  Measured on B200: a warp's plane 330 (REAL) / 480 (COMPLEX) cycles
 // with several warps on the scheduler, 900 / 1200 alone; 0.7 cycles a packet; 2300
 // for the exchange itself.
-// Best of the cuts tried, and this model's: REAL 32^3 2.16 / 2.23 us a step, 64^3
-// 3.53 / 3.53, 96^3 7.5 / 7.5; COMPLEX 64^3 4.37 / 4.40, 96^3 9.2 / 9.2.
+// When the model was fitted, the best of the cuts tried and this model's: REAL 32^3
+// 2.16 / 2.23 us a step, 64^3 3.53 / 3.53, 96^3 7.5 / 7.5; COMPLEX 64^3 4.37 / 4.40,
+// 96^3 9.2 / 9.2.  The model's cuts now take 1.87, 3.23, 6.57; 3.87, 8.26 us, the
+// tile kernel launched once a step 7.2, 8.7, 13.3; 9.3, 20.7.
 //
 // plans[c]: the cheapest cut of at most c blocks (c = 0: none), for c up to 148.
 static const std::vector<ResidentPlan>& resident_plans(int level, int N) {

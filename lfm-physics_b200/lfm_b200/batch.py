@@ -3,8 +3,11 @@
 The reference runs a parameter sweep one ``Simulation`` after another
 (lfm/sweep.py:52-82: deep-copy the config, build, run, read metrics).  Small
 lattices leave most of a B200 idle that way.  ``BatchedLattices`` holds every
-lattice of a sweep resident in one device arena and advances all of them with
-one persistent kernel launch per step (lfm_batch_step): the CTAs take
+lattice of a sweep resident in one device arena.  ``evolve`` holds them on chip,
+as many side by side as the SMs take, and runs a wave's steps in one launch
+(lfm_batch_run).  Where one does not fit (REAL above 108^3, COMPLEX above 96^3),
+under a tuning of the tile kernel and for runs of under four steps it advances
+all of them with one persistent kernel launch per step (lfm_batch_step): the CTAs take
 (lattice, row tile, plane chunk) items from a work list grouped by lattice
 shape (the sweep's shapes at 256 threads run with their geometry fixed at
 compile time) and sorted by cost within each group, each marched exactly like
@@ -12,8 +15,8 @@ the fused single-lattice kernel, so every lattice's result is bit-for-bit the
 one ``Evolver`` gives for it alone.
 
 Lattices may differ in N (multiples of 4), level (REAL or COMPLEX), sponge
-and every coupling constant.  ``evolve`` replays a captured CUDA graph of a
-block of steps.  Field accessors take the lattice index first and follow the
+and every coupling constant.  Single steps are replayed as a captured CUDA graph
+of a block of steps.  Field accessors take the lattice index first and follow the
 reference ``Evolver``'s semantics (set_psi_real sets current and previous,
 get_psi_real_prev returns the sponge-damped previous field).
 """
@@ -33,7 +36,7 @@ _ALIGN = 64  # floats: every slot starts on a 256-byte boundary
 
 
 class BatchedLattices:
-    """REAL / COMPLEX lattices of mixed sizes, one persistent launch per step."""
+    """REAL / COMPLEX lattices of mixed sizes, stepped together."""
 
     graph_block = 16
     """Steps per captured CUDA graph (an even number)."""

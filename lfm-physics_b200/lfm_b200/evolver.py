@@ -215,7 +215,8 @@ class Evolver:
     # time loop (evolver.py:137-180)
     # ------------------------------------------------------------------
     use_graphs = True
-    """Replay captured CUDA graphs of two steps when evolve() has no per-step host work."""
+    """When evolve() has no per-step host work: on-chip runs where the lattice fits, else
+    captured CUDA graphs of two steps."""
     hook_block = 32
     """Steps per captured graph when evolve() runs device hooks (even: parity returns)."""
 
