@@ -166,13 +166,17 @@ def set_step_path(path: int) -> None:
 
 
 def run_workspace(level: int, N: int, device):
-    """Zeroed workspace of lfm_leapfrog_run_f32 for one lattice; empty if it does not fit."""
+    """Zeroed workspace of lfm_leapfrog_run_f32 for one lattice; empty if the lattice does
+    not fit on chip or there is no memory for it (both take single steps)."""
     import torch
 
     n = ctypes.c_longlong(0)
     with torch.cuda.device(device):
         call("lfm_leapfrog_run_words", int(level), int(N), ctypes.byref(n))
-    return torch.zeros(n.value, dtype=torch.int32, device=device)
+    try:
+        return torch.zeros(n.value, dtype=torch.int32, device=device)
+    except torch.OutOfMemoryError:
+        return torch.empty(0, dtype=torch.int32, device=device)
 
 
 def run_steps(name: str, *args) -> bool:

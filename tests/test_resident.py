@@ -133,6 +133,24 @@ def test_forced_path_and_tile_keep_the_single_steps(be):
 
 
 @pytest.mark.gpu
+def test_no_memory_for_the_workspace_keeps_the_single_steps(be, monkeypatch):
+    import torch
+
+    a, b = _evolver(COMPLEX, 16, 3, be), _evolver(COMPLEX, 16, 3, be)
+
+    def no_memory(*args, **kwargs):
+        raise torch.OutOfMemoryError("planted")
+
+    with monkeypatch.context() as m:
+        m.setattr(torch, "zeros", no_memory)
+        a.evolve(9)
+    assert a._run_sync.numel() == 0
+    b.use_graphs = False
+    b.evolve(9)
+    _same(a, b)
+
+
+@pytest.mark.gpu
 def test_two_lattices_on_two_streams(be):
     """Launches that wait on one another's CTAs only: two at a time do not mix."""
     import torch
