@@ -90,6 +90,22 @@ def test_other_filter_parameters_get_their_own_table(be):
         assert np.abs(got - ref).max() <= SA_REL_TOL * np.abs(ref).max(), (gamma, d)
 
 
+def test_many_filter_constants_give_the_same_bits_with_and_without_a_table(be):
+    """The first pairs of constants keep a table, later ones work the factors out: two
+    contexts that meet the pairs in opposite orders, so each pair is solved both ways."""
+    from lfm_b200 import B200Backend
+
+    N = 20
+    pr, pi = _packets(N, 7)
+    pairs = [(0.1 + 0.05 * k, 4.9 - 0.2 * k) for k in range(17)]
+    one, other = B200Backend(be.device), B200Backend(be.device)
+    a = {p: _sa(one, pr, pi, N, 1, *p) for p in pairs}
+    b = {p: _sa(other, pr, pi, N, 1, *p) for p in reversed(pairs)}
+    for p in pairs:
+        assert a[p].tobytes() == b[p].tobytes(), p
+    assert a[pairs[0]].tobytes() != a[pairs[1]].tobytes()
+
+
 def test_color_evolver_64_with_split_transform_against_oracle(be):
     """The resident COLOR Evolver at 64^3 with S_a every step (split transform) stays within
     the COLOR tolerance of the oracle's float32 steps (NumPy S_a) over 20 steps."""
