@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "lfm_kernels.h"
+#include "lfm_launch.h"
 #include "lfm_queue.cuh"
 #include "lfm_resident.h"
 
@@ -595,18 +596,10 @@ __global__ void __launch_bounds__(THREADS, 1)
 
 template <int LEVEL, bool EVEN, int THREADS, int LATTICES>
 cudaError_t launch(const Wave<LATTICES>& w, int threads, int smem, cudaStream_t stream) {
-  static std::mutex mu;
-  static int granted = 0;
+  static SmemGrant grant;
   const auto kernel = resident_kernel<LEVEL, EVEN, THREADS, LATTICES>;
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    if (smem > granted) {
-      cudaError_t e =
-          cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      if (e != cudaSuccess) return e;
-      granted = smem;
-    }
-  }
+  const cudaError_t e = grant.raise((const void*)kernel, smem);
+  if (e != cudaSuccess) return e;
   void* args[] = {const_cast<Wave<LATTICES>*>(&w)};
   return cudaLaunchCooperativeKernel((const void*)kernel, dim3(w.first[w.count]), dim3(threads),
                                      args, (size_t)smem, stream);

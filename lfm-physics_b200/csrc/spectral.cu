@@ -30,6 +30,7 @@
 // (k = 2 pi fftfreq(N)); k^2 depends only on the magnitudes of the integer
 // frequencies, so (N/2+1)^3 entries cover the spectrum.
 #include "lfm_kernels.h"
+#include "lfm_launch.h"
 
 #include <cmath>
 
@@ -387,13 +388,9 @@ cudaError_t launch_xpass(float2* spec, const float* table, const float2* tw,
                          cudaStream_t stream) {
   constexpr int N = N1 * N2;
   constexpr int smem = (N + N * TW) * (int)sizeof(float2);
-  static bool granted = false;  // the attribute is per function and process
-  if (!granted) {
-    cudaError_t e = cudaFuncSetAttribute(helmholtz_xpass_kernel<N1, N2, TW>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    granted = true;
-  }
+  static SmemGrant grant;
+  const cudaError_t e = grant.raise((const void*)helmholtz_xpass_kernel<N1, N2, TW>, smem);
+  if (e != cudaSuccess) return e;
   const int64_t W = (int64_t)N * (N / 2 + 1);
   const int64_t tiles = 3 * (W / TW);
   helmholtz_xpass_kernel<N1, N2, TW><<<(unsigned)tiles, N1 * TW, smem, stream>>>(spec, table,

@@ -27,11 +27,11 @@
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
-#include <mutex>
 
 #include "lfm_cells.cuh"
 #include "lfm_batch.h"
 #include "lfm_kernels.h"
+#include "lfm_launch.h"
 #include "lfm_queue.cuh"
 #include "lfm_tune.h"
 
@@ -1409,27 +1409,12 @@ cudaError_t kernel_regs(K kernel, int* regs) {
   return e;
 }
 
-// Raises the kernel's dynamic shared-memory limit to what the launch needs
-// (within the device's opt-in limit less its static shared memory) and launches.
+// Raises the kernel's dynamic shared-memory limit to what the launch needs and launches.
 template <typename K>
-cudaError_t launch_kernel(K kernel, int* granted, std::mutex* mu, const TmaParams& P,
-                          const Choice& ch, cudaStream_t stream) {
-  {
-    std::lock_guard<std::mutex> lk(*mu);
-    if (ch.smem > *granted) {
-      int dev = 0, optin = 0;
-      cudaError_t e = cudaGetDevice(&dev);
-      if (e == cudaSuccess)
-        e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-      cudaFuncAttributes fa{};
-      if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, kernel);
-      if (e != cudaSuccess) return e;
-      if (ch.smem + (int)fa.sharedSizeBytes > optin) return cudaErrorNotSupported;
-      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ch.smem);
-      if (e != cudaSuccess) return e;
-      *granted = ch.smem;
-    }
-  }
+cudaError_t launch_kernel(K kernel, SmemGrant& grant, const TmaParams& P, const Choice& ch,
+                          cudaStream_t stream) {
+  const cudaError_t e = grant.raise((const void*)kernel, ch.smem);
+  if (e != cudaSuccess) return e;
   const int JT = P.N / P.TJ;
   const int planes = P.a.slab ? P.a.i_hi - P.a.i_lo : P.N;
   const int chunks = (planes + P.IC - 1) / P.IC;
@@ -1439,8 +1424,7 @@ cudaError_t launch_kernel(K kernel, int* granted, std::mutex* mu, const TmaParam
 
 template <int LEVEL, int V, bool QUEUE, int MODE>
 struct KernelSlot {
-  static std::mutex mu;
-  static int granted;
+  static SmemGrant grant;
   static auto fn() {
     if constexpr (QUEUE)
       return tma_queue_kernel<LEVEL, V, MODE>;
@@ -1449,25 +1433,20 @@ struct KernelSlot {
   }
 };
 template <int LEVEL, int V, bool QUEUE, int MODE>
-std::mutex KernelSlot<LEVEL, V, QUEUE, MODE>::mu;
-template <int LEVEL, int V, bool QUEUE, int MODE>
-int KernelSlot<LEVEL, V, QUEUE, MODE>::granted = 0;
+SmemGrant KernelSlot<LEVEL, V, QUEUE, MODE>::grant;
 
 // Compile-time tiles for the headline sizes (resident layout); MODE kComp:
 // the compensated (Delta-form) step on the same tile.
 template <int LEVEL, int V, int N, int TJ, int S, int MODE = kPlain, bool SLAB = false>
 struct FixedSlot {
-  static std::mutex mu;
-  static int granted;
+  static SmemGrant grant;
   static auto fn() {
     using F = QFields<LEVEL, MODE>;
     return tma_queue_kernel<LEVEL, V, MODE, GeomCT<N, TJ, F::ns, S, SLAB, F::np>>;
   }
 };
 template <int LEVEL, int V, int N, int TJ, int S, int MODE, bool SLAB>
-std::mutex FixedSlot<LEVEL, V, N, TJ, S, MODE, SLAB>::mu;
-template <int LEVEL, int V, int N, int TJ, int S, int MODE, bool SLAB>
-int FixedSlot<LEVEL, V, N, TJ, S, MODE, SLAB>::granted = 0;
+SmemGrant FixedSlot<LEVEL, V, N, TJ, S, MODE, SLAB>::grant;
 
 // The compile-time tiles: step form, level, cells per lane, N, rows, stages.
 // The compensated step has one at the throughput size; split chi at 256^3 and
@@ -1500,7 +1479,7 @@ const FixedTile* fixed_tile(int mode, int level, int V, int N) {
 template <int LEVEL, int V, int N, int TJ, int MODE = kPlain, bool SLAB = false>
 cudaError_t launch_fixed(TmaParams& P, const Choice& ch, cudaStream_t stream) {
   using Slot = FixedSlot<LEVEL, V, N, TJ, fixed_stages(MODE, LEVEL, V, N, TJ), MODE, SLAB>;
-  return launch_kernel(Slot::fn(), &Slot::granted, &Slot::mu, P, ch, stream);
+  return launch_kernel(Slot::fn(), Slot::grant, P, ch, stream);
 }
 
 // Shared memory of the sponge table of the compile-time tiles: count entries
@@ -1556,10 +1535,8 @@ bool try_fixed(TmaParams& P, const Choice& ch, cudaStream_t stream, cudaError_t*
 // The barrier kernel's compile-time tiles.
 template <int N, int TJ, int S>
 cudaError_t launch_color(TmaParams& P, const Choice& ch, cudaStream_t stream) {
-  static std::mutex mu;
-  static int granted = 0;
-  return launch_kernel(tma_step_kernel<LFM_COLOR, 2, ColorCT<N, TJ, S>>, &granted, &mu, P, ch,
-                       stream);
+  static SmemGrant grant;
+  return launch_kernel(tma_step_kernel<LFM_COLOR, 2, ColorCT<N, TJ, S>>, grant, P, ch, stream);
 }
 
 bool try_color(TmaParams& P, const Choice& ch, cudaStream_t stream, cudaError_t* err) {
@@ -1654,7 +1631,7 @@ cudaError_t plan_and_launch(TmaParams& P, const TileConfig* forced, bool any_til
   }
   if (!any_tile && !run_time_tile_pays<LEVEL, QUEUE, MODE>(P, ch)) return cudaErrorNotSupported;
   tune_record(LEVEL, P.N, used);
-  return launch_kernel(Slot::fn(), &Slot::granted, &Slot::mu, P, ch, stream);
+  return launch_kernel(Slot::fn(), Slot::grant, P, ch, stream);
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -1786,28 +1763,6 @@ cudaError_t launch_tma_step(const StepArgs& a, bool any_tile, cudaStream_t strea
 
 
 // ---- batch launcher -------------------------------------------------------------
-namespace {
-std::mutex g_batch_mu;
-int g_batch_granted[2] = {0, 0};  // dynamic shared memory granted to the two batch kernels
-
-template <typename K>
-cudaError_t grant_smem(K kernel, int smem, int* granted) {
-  std::lock_guard<std::mutex> lk(g_batch_mu);
-  if (smem <= *granted) return cudaSuccess;
-  int dev = 0, optin = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess)
-    e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  cudaFuncAttributes fa{};
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, kernel);
-  if (e != cudaSuccess) return e;
-  if (smem + (int)fa.sharedSizeBytes > optin) return cudaErrorNotSupported;
-  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess) *granted = smem;
-  return e;
-}
-}  // namespace
-
 cudaError_t batch_kernel_regs(int* regs) {
   // the larger of the two variants' demands
   cudaFuncAttributes fa{}, fb{};
@@ -1822,7 +1777,8 @@ cudaError_t launch_batch_step(const BatchParams& B, int threads, int smem, int g
   if (B.nitems == 0) return cudaSuccess;
   const bool tab = B.tab_off >= 0;
   auto kernel = tab ? tma_batch_kernel<1> : tma_batch_kernel<-1>;
-  cudaError_t e = grant_smem(kernel, smem, &g_batch_granted[tab ? 1 : 0]);
+  static SmemGrant grant[2];
+  const cudaError_t e = grant[tab ? 1 : 0].raise((const void*)kernel, smem);
   if (e != cudaSuccess) return e;
   kernel<<<grid, threads, smem, stream>>>(B);
   return cudaGetLastError();

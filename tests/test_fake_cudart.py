@@ -1,0 +1,113 @@
+"""The library's launch code on a CUDA runtime without a GPU (fake_cudart.cpp): two devices
+in one process, and cooperative launches that are refused.  The library's own objects are
+linked against it; a launch is checked and counted, and runs nothing."""
+
+from __future__ import annotations
+
+import ctypes
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import ROOT
+from lfm_b200 import _lib
+from lfm_b200.build import LIB_DIR, build_library, sources
+from lfm_b200.mask import MaskTable
+
+REAL, COMPLEX, COLOR = 0, 1, 2
+STEP = (4e-4, 1 / 63, 0.0, 19.0, 0.0)  # dt2, kappa, lambda_self, chi0, e0_sq
+
+
+@pytest.fixture(scope="module")
+def fake_path(tmp_path_factory):
+    build_library()
+    objs = [LIB_DIR / "obj" / f"{s.stem}.o" for s in sources()]
+    if not all(o.exists() for o in objs):
+        build_library(force=True)
+    out = tmp_path_factory.mktemp("fake") / "liblfm_fake.so"
+    subprocess.check_call(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-Wl,-Bsymbolic",
+                           "-I/usr/local/cuda/include", "-o", str(out),
+                           str(ROOT / "tests" / "fake_cudart.cpp"), *map(str, objs)])
+    return out
+
+
+@pytest.fixture
+def fake(fake_path, monkeypatch):
+    """The linked library, in the package's place, as a process finds it at its start."""
+    lib = ctypes.CDLL(str(fake_path))
+    for name, args in _lib._SIGNATURES.items():
+        getattr(lib, name).argtypes = args
+    lib.lfm_strerror.restype = lib.lfm_last_error_detail.restype = ctypes.c_char_p
+    monkeypatch.setattr(_lib, "_lib", lib)
+    lib.fake_reset()
+    return lib
+
+
+class Lattice:
+    """Host buffers in the place of a lattice's device memory."""
+
+    def __init__(self, level, N):
+        self.level, self.N = level, N
+        per = 3 if level == COLOR else 1
+        self.bufs = [np.zeros(per * N**3 + 4, np.float32) for _ in range(6)]
+        self.p = [(b.ctypes.data + 15) & ~15 for b in self.bufs]
+        self.pr, self.pi, self.chi = self.p[:2], self.p[2:4] if level else (None, None), self.p[4:]
+        self.table = MaskTable.for_lattice(N, 0.3)
+        self.t = np.ascontiguousarray(self.table.table, np.float32)
+        self.mask = (self.t.ctypes.data, ctypes.byref(self.table.desc))
+        words = ctypes.c_longlong()
+        _lib.call("lfm_leapfrog_run_words", min(level, 1), N, ctypes.byref(words))
+        self.sync = np.zeros(words.value + 4, np.int32)
+
+    def run(self, steps=4):
+        return _lib.run_steps("lfm_leapfrog_run_f32", self.level, steps, *self.pr, *self.pi,
+                              *self.chi, *self.mask, 0, self.N, *STEP, 0.1, None,
+                              (self.sync.ctypes.data + 15) & ~15, None)
+
+    def step(self):
+        if self.level == REAL:
+            _lib.call("lfm_leapfrog_real_f32", *self.pr, *self.chi, *self.mask, 0, self.N, *STEP,
+                      None)
+        else:
+            _lib.call("lfm_leapfrog_color_f32", *self.pr, *self.pi, *self.chi, *self.mask, 0,
+                      self.N, *STEP, *([0.1] * 5), None, None)
+
+    def desc(self):
+        d = _lib.LatticeDesc()
+        d.N, d.level = self.N, self.level
+        for s in range(2):
+            d.psi_r[s], d.psi_i[s], d.chi[s] = self.pr[s], self.pi[s], self.chi[s]
+        d.mask_table, d.lut = self.t.ctypes.data, self.table.desc
+        d.dt2, d.kappa, d.lambda_self, d.chi0, d.e0_sq = STEP
+        return d
+
+
+def batch(lattices):
+    descs = (_lib.LatticeDesc * len(lattices))(*[x.desc() for x in lattices])
+    h = ctypes.c_void_p()
+    _lib.call("lfm_batch_create", descs, len(lattices), None, ctypes.byref(h))
+    return h
+
+
+def solve_sa(N):
+    ctx = ctypes.c_void_p()
+    _lib.call("lfm_context_create", ctypes.byref(ctx))
+    e, s = (np.zeros(3 * N**3, np.float32) for _ in range(2))
+    _lib.call("lfm_helmholtz_sa_from_energy_f32", ctx, e.ctypes.data, s.ctypes.data, N, 0.1, 4.9,
+              None)
+
+
+@pytest.mark.parametrize("what", ["run", "color", "fused", "batch", "s_a"])
+def test_shared_memory_limits_are_raised_on_every_device(fake, what):
+    """The limit of a kernel's dynamic shared memory belongs to the device: what a process
+    launches on its first GPU it can launch on its second."""
+    call = {"run": lambda: Lattice(REAL, 32).run(), "color": Lattice(COLOR, 128).step,
+            "fused": Lattice(REAL, 128).step,
+            "batch": lambda: _lib.call("lfm_batch_step", batch([Lattice(REAL, 96)]), 0, 0, None),
+            "s_a": lambda: solve_sa(512)}[what]
+    for device in (0, 1, 0):
+        fake.cudaSetDevice(device)
+        before = fake.fake_launches()
+        call()
+        assert fake.fake_launches() > before and fake.fake_refusals() == 0
