@@ -165,9 +165,9 @@ int lfm_leapfrog_complex_f32(const float* psi_r, float* psi_r_prev_io, const flo
  * COMPLEX, chi; apart from the slots) that the time level made by step s is stored
  * to as well; null entries are skipped (all of a step's or none).
  * Returns LFM_ERR_UNSUPPORTED (nothing launched) when the lattice does not fit
- * on chip, steps < 2, a slot of an N % 4 == 0 lattice is not 16-byte aligned, or a
- * step path or tile was forced with lfm_set_step_path / lfm_tune_set: the
- * caller then takes the single steps. */
+ * on chip or has no room there beside what the context may use, steps < 2, a slot of an
+ * N % 4 == 0 lattice is not 16-byte aligned, or a step path or tile was forced with
+ * lfm_set_step_path / lfm_tune_set: the caller then takes the single steps. */
 int lfm_leapfrog_run_f32(int level, int steps, float* psi_r_s0, float* psi_r_s1,
                          float* psi_i_s0, float* psi_i_s1, float* chi_s0, float* chi_s1,
                          const float* mask_table, const lfm_mask_lut* lut, int damp_prev, int N,
@@ -417,7 +417,8 @@ typedef struct lfm_batch lfm_batch;
 /* `steps` steps of every lattice with the state held on chip, waves of lattices one
  * after another (the same bits as `steps` calls of lfm_batch_step; the current fields
  * are then in slot parity + steps mod 2).  LFM_ERR_UNSUPPORTED, with nothing launched,
- * when a lattice does not fit on chip, steps < 2 or a step path is forced. */
+ * when a lattice does not fit on chip or a wave has no room there, steps < 2 or a step
+ * path is forced. */
 int lfm_batch_run(lfm_batch* batch, int steps, int parity, int damp_prev, void* stream);
 
 

@@ -709,6 +709,14 @@ int lfm_leapfrog_run_plan(int level, int N, int sms, int* plan) {
 
 namespace {
 
+// Whether a run's launch was refused because its blocks cannot all be resident at once
+// (fewer SMs for this context than the device has): the lattice takes single steps.
+bool no_room_for_run(cudaError_t e) {
+  if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported) return false;
+  cudaGetLastError();
+  return true;
+}
+
 // Checks and launches an on-chip run.  cur / prev: (psi_r, psi_i, chi) at the current
 // and previous time level; even / odd: where the last two time levels go, or null.
 int run_on_chip(int level, int steps, const float* const cur[3], const float* const prev[3],
@@ -765,6 +773,7 @@ int run_on_chip(int level, int steps, const float* const cur[3], const float* co
   a.sync = sync;
   a.packets = reinterpret_cast<ulonglong2*>(sync + 4);
   e = lfm::launch_resident(a, static_cast<cudaStream_t>(stream));
+  if (no_room_for_run(e)) return fail(LFM_ERR_UNSUPPORTED, "run: %s", cudaGetErrorString(e));
   if (e != cudaSuccess) return cuda_fail(e, "resident run launch");
   return LFM_OK;
 }
@@ -1679,6 +1688,7 @@ int lfm_batch_run(lfm_batch* batch, int steps, int parity, int damp_prev, void* 
   int* status = nullptr;
   int rc = status_word(&status);
   if (rc) return rc;
+  bool first = true;
   for (const lfm::ResidentWavePlan& w : batch->waves) {
     std::vector<lfm::ResidentArgs> args(w.lattices.size());
     uint32_t* at = batch->d_sync + 4;
@@ -1706,7 +1716,11 @@ int lfm_batch_run(lfm_batch* batch, int steps, int parity, int damp_prev, void* 
     }
     cudaError_t e = lfm::launch_resident_wave(args.data(), (int)args.size(),
                                               static_cast<cudaStream_t>(stream));
+    // the waves come in order of their blocks: nothing has run if one is refused
+    if (first && no_room_for_run(e))
+      return fail(LFM_ERR_UNSUPPORTED, "batch run: %s", cudaGetErrorString(e));
     if (e != cudaSuccess) return cuda_fail(e, "batch run launch");
+    first = false;
   }
   return LFM_OK;
 }

@@ -58,8 +58,8 @@ struct ResidentWavePlan {
 };
 constexpr int kWaveLattices = 32;  // at most, in a wave
 
-// The waves that run `count` lattices on chip one wave after another, and the model's
-// cycles of a step through all of them; false if a lattice does not fit or its N is odd.
+// The waves that run `count` lattices on chip one wave after another, those of the most
+// blocks first, and the model's cycles of a step through all of them; false if a lattice does not fit or its N is odd.
 bool resident_waves(const int* level, const int* N, int count, int sms,
                     std::vector<ResidentWavePlan>* waves, double* cycles);
 

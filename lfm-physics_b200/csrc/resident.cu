@@ -769,6 +769,11 @@ bool resident_waves(const int* level, const int* N, int count, int sms,
     }
     if (!idx.empty()) *cycles += pack_level(N, idx, lv, sms, waves);
   }
+  // the most blocks first, so that a launch the device has no room for is the first one
+  std::stable_sort(waves->begin(), waves->end(),
+                   [](const ResidentWavePlan& a, const ResidentWavePlan& b) {
+                     return a.blocks > b.blocks;
+                   });
   return true;
 }
 

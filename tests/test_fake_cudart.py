@@ -111,3 +111,29 @@ def test_shared_memory_limits_are_raised_on_every_device(fake, what):
         before = fake.fake_launches()
         call()
         assert fake.fake_launches() > before and fake.fake_refusals() == 0
+
+
+def test_a_refused_run_leaves_the_lattice_to_single_steps(fake):
+    """Blocks that cannot all be resident at once (a context with a part of the SMs): the
+    run answers that it is not supported, and has launched nothing."""
+    lat = Lattice(REAL, 32)
+    fake.fake_free_sms(60)
+    assert lat.run() is False
+    assert fake.fake_launches() == 0 and fake.fake_refusals() == 1 and fake.fake_last_error() == 0
+    lat.step()
+    fake.fake_free_sms(148)
+    assert lat.run() is True
+
+
+@pytest.mark.parametrize("sizes", [[(8, REAL), (96, COMPLEX)], [(96, REAL), (8, COMPLEX)]])
+def test_a_refused_wave_leaves_the_batch_to_single_steps(fake, sizes):
+    """A batch's largest wave is refused before any other has run."""
+    lats = [Lattice(level, n) for n, level in sizes]
+    h = batch(lats)
+    before = fake.fake_launches()
+    fake.fake_free_sms(100)
+    assert _lib.run_steps("lfm_batch_run", h, 4, 0, 0, None) is False
+    assert fake.fake_launches() == before and fake.fake_last_error() == 0
+    _lib.call("lfm_batch_step", h, 0, 0, None)
+    fake.fake_free_sms(148)
+    assert _lib.run_steps("lfm_batch_run", h, 4, 0, 0, None) is True
