@@ -1301,6 +1301,7 @@ __global__ void __launch_bounds__(512, 1) tma_batch_kernel(const __grid_constant
 // ---- host side -------------------------------------------------------------------
 struct Choice {
   int TJ = 0, S = 0, IC = 0, threads = 0, smem = 0;
+  int warps = 0;  // resident on an SM
 };
 
 // Dynamic shared memory a configuration may use: the 227 KB opt-in limit
@@ -1373,6 +1374,7 @@ Choice choose(int level, int N, int V, int ns, int np, bool queue, int max_threa
   const int ctas = std::max(1, std::min(std::min((228 * 1024) / (best.smem + 1024),
                                                  2048 / best.threads),
                                         65536 / std::max(1, regs * best.threads)));
+  best.warps = ctas * best.threads / 32;
   if (forced && forced->ic > 0) {
     best.IC = std::min(forced->ic, planes);
   } else {
@@ -1547,21 +1549,44 @@ bool try_color(TmaParams& P, const Choice& ch, cudaStream_t stream, cudaError_t*
 }
 
 // Whether a run-time tile is still the faster kernel where the marching kernel of
-// step_march.cu runs too.  With its strides in registers the ring's march is slower
-// than that kernel's loads through L1 at every COMPLEX size (us a step, tile against
-// march: 104^3 29.3 / 19.9, 160^3 82.6 / 66.6, 288^3 570 / 336, 384^3 962 / 759), for
-// split chi (REAL 96^3 30.5 / 13.6, 160^3 93.7 / 55.8, COMPLEX 128^3 46.1 / 39.2), the
-// compensated step (REAL 128^3 25.9 / 22.7) and the protocol's streamed mask (COMPLEX
-// 96^3 25.2 / 21.8, REAL 128^3 25.8 / 23.1).  The plain REAL step keeps its tile where
-// it fills a CTA of 384 threads or more on a lattice of 192^3 or more (192^3 61.5 /
-// 66.2, 224^3 92.4 / 96.7, 240^3 113 / 125, 384^3 443 / 450); smaller ones lose as well
-// (112^3 19.9 / 15.9, 144^3 43.5 / 26.2, 176^3 65.8 / 48.5, 288^3 253 / 194).
-template <int LEVEL, bool QUEUE, int MODE>
+// step_march.cu (below its smallest sizes: the direct kernel) runs too.  us a step, tile /
+// march, with every edge that has a tile measured from 112^3 to 512^3 and 640^3, 768^3 and
+// 1024^3 beside them.
+//
+// With its strides in registers the ring's march is slower than that kernel's loads
+// through L1 at every COMPLEX size (104^3 28.1 / 18.4, 160^3 81.9 / 66.2, 288^3 573 / 336,
+// 384^3 957 / 759, 1024^3 14375 / 14239) and for split chi (REAL 96^3 29.5 / 12.3, 160^3
+// 92.0 / 54.7, 640^3 5066 / 3163; COMPLEX 128^3 44.9 / 37.8; only COMPLEX 240^3 is the
+// other way, 263 / 269).  What a tile needs to keep up is warps on the SM:
+//
+// - the plain REAL step from 192^3 on, with CTAs of 384 threads or more (192^3 60.1 /
+//   66.2, 224^3 92.1 / 96.7, 240^3 113 / 125; but 176^3 65.8 / 48.5, 288^3 254 / 194 with 9
+//   warps, 352^3 369 / 350 with 11).
+// - the REAL step with a streamed mask, which stores the previous fields too, from 160^3
+//   with 11 warps or more (160^3 36.4 / 43.0, 192^3 60.4 / 71.2, 256^3 129 / 152, 352^3
+//   363 / 386, 512^3 938 / 1153, 1024^3 7406 / 9104; but 128^3 22.1 / 19.3, 144^3 36.1 /
+//   31.6, 288^3 246 / 213 with 9); the COMPLEX one with CTAs of 480 or 512 threads (128^3
+//   35.8 / 37.4, 240^3 215 / 225, 256^3 237 / 250, 512^3 1747 / 1863; but 192^3 126 / 113
+//   with 384, 224^3 186 / 166 with 448).
+// - the compensated step with CTAs as large (REAL 240^3 139 / 147, 256^3 149 / 165, 480^3
+//   965 / 1042; but 128^3 24.7 / 21.3, 224^3 117 / 114 with 448; COMPLEX, 512 threads:
+//   256^3 277 / 285, 512^3 2071 / 2187; but 128^3 43.4 / 36.6, 480^3 1851 / 1808).
+// - COLOR with 12 warps or more: 192^3 286 / 323, 208^3 404 / 415, 224^3 437 / 513; but
+//   144^3 164 / 141 and 288^3 1272 / 1093 with 9, 160^3 210 / 193 with 10.  Without S_a or
+//   a mask from 112^3 (61.3 / 61.3; 96^3 38.0 / 35.2), with either from 80^3 (with S_a
+//   61.4 / 62.7, 112^3 148 / 157; masked 23.6 / 24.6, 112^3 63.7 / 72.9).
+//
+// Below 32^3 (COLOR 45^3) the direct kernel is the other one, and far ahead (REAL 16^3 6.3 /
+// 2.7, COMPLEX 24^3 6.9 / 3.3, COLOR 40^3 11.5 / 6.5).
+template <int LEVEL, int MODE>
 bool run_time_tile_pays(const TmaParams& P, const Choice& ch) {
-  // COLOR: 72^3 33.3 / 23.3, 144^3 214 / 156, 192^3 372 / 346 with 192 to 288 threads a
-  // CTA; 240^3 573 / 663 with 480
-  if (LEVEL == LFM_COLOR) return ch.threads >= 448;
-  return LEVEL == LFM_REAL && MODE == kPlain && P.pf_mask < 0 && P.N >= 192 && ch.threads >= 384;
+  const bool masked = P.a.mask != nullptr;
+  if (LEVEL == LFM_COLOR) return ch.warps >= 12 && P.N >= (P.a.sa || masked ? 80 : 112);
+  if (MODE == kComp) return P.N >= 160 && ch.threads >= (LEVEL == LFM_REAL ? 480 : 512);
+  if (MODE == kSplit) return false;
+  if (LEVEL == LFM_REAL)
+    return masked ? P.N >= 160 && ch.warps >= 11 : P.N >= 192 && ch.threads >= 384;
+  return masked && P.N >= 128 && ch.threads >= 480;
 }
 
 // any_tile: the caller asks for the fused kernel, whichever is faster.
@@ -1629,7 +1654,7 @@ cudaError_t plan_and_launch(TmaParams& P, const TileConfig* forced, bool any_til
       return ce;
     }
   }
-  if (!any_tile && !run_time_tile_pays<LEVEL, QUEUE, MODE>(P, ch)) return cudaErrorNotSupported;
+  if (!any_tile && !run_time_tile_pays<LEVEL, MODE>(P, ch)) return cudaErrorNotSupported;
   tune_record(LEVEL, P.N, used);
   return launch_kernel(Slot::fn(), Slot::grant, P, ch, stream);
 }

@@ -12,7 +12,7 @@
 
 namespace {
 constexpr int kSms = 148, kOptin = 227 * 1024, kDefault = 48 * 1024;
-int device = 0, free_sms = kSms, launches = 0, refusals = 0;
+int device = 0, free_sms = kSms, launches = 0, refusals = 0, shared = 0;
 cudaError_t last = cudaSuccess;
 std::map<std::pair<int, const void*>, int> limit;  // raised limits: (device, kernel)
 struct Config {
@@ -32,6 +32,7 @@ cudaError_t launch(const void* kernel, dim3 grid, size_t smem, bool cooperative)
   if (smem > (size_t)(it == limit.end() ? kDefault : it->second)) e = cudaErrorInvalidValue;
   if (cooperative && (int)grid.x > free_sms) e = cudaErrorCooperativeLaunchTooLarge;
   ++(e == cudaSuccess ? launches : refusals);
+  shared = (int)smem;
   return ret(e);
 }
 }  // namespace
@@ -39,6 +40,7 @@ cudaError_t launch(const void* kernel, dim3 grid, size_t smem, bool cooperative)
 extern "C" {
 int fake_launches() { return launches; }
 int fake_refusals() { return refusals; }
+int fake_dynamic_smem() { return shared; }  // of the last launch
 int fake_last_error() { return last; }
 void fake_free_sms(int n) { free_sms = n; }
 void fake_reset() {
@@ -85,7 +87,7 @@ cudaError_t cudaGetLastError() { return std::exchange(last, cudaSuccess); }
 const char* cudaGetErrorString(cudaError_t) { return "fake"; }
 cudaError_t cudaFuncGetAttributes(cudaFuncAttributes* a, const void*) {
   memset(a, 0, sizeof *a);
-  a->numRegs = 64;
+  a->numRegs = 128;
   a->sharedSizeBytes = 128;
   return cudaSuccess;
 }

@@ -69,9 +69,30 @@ class Lattice:
         if self.level == REAL:
             _lib.call("lfm_leapfrog_real_f32", *self.pr, *self.chi, *self.mask, 0, self.N, *STEP,
                       None)
+        elif self.level == COMPLEX:
+            _lib.call("lfm_leapfrog_complex_f32", *self.pr, *self.pi, *self.chi, *self.mask, 0,
+                      self.N, *STEP, 0.1, None)
         else:
             _lib.call("lfm_leapfrog_color_f32", *self.pr, *self.pi, *self.chi, *self.mask, 0,
                       self.N, *STEP, *([0.1] * 5), None, None)
+
+    def masked_step(self):
+        """The protocol's step: a mask beside the fields, every output apart."""
+        n = self.N**3
+        f = [np.zeros(n + 4, np.float32) for _ in range(13)]
+        p = [(b.ctypes.data + 15) & ~15 for b in f]
+        if self.level == REAL:
+            _lib.call("lfm_step_real_f32", *p[:9], self.N, *STEP, None)
+        else:
+            _lib.call("lfm_step_complex_f32", *p, self.N, *STEP, 0.1, None)
+
+    def comp_step(self):
+        f = [np.zeros(self.N**3 + 4, np.float32) for _ in range(9)]
+        p = [(b.ctypes.data + 15) & ~15 for b in f]
+        if self.level == REAL:
+            _lib.call("lfm_leapfrog_real_comp_f32", *p[:6], *self.mask, self.N, *STEP, None)
+        else:
+            _lib.call("lfm_leapfrog_complex_comp_f32", *p, *self.mask, self.N, *STEP, 0.1, None)
 
     def desc(self):
         d = _lib.LatticeDesc()
@@ -137,3 +158,18 @@ def test_a_refused_wave_leaves_the_batch_to_single_steps(fake, sizes):
     _lib.call("lfm_batch_step", h, 0, 0, None)
     fake.fake_free_sms(148)
     assert _lib.run_steps("lfm_batch_run", h, 4, 0, 0, None) is True
+
+
+@pytest.mark.parametrize("level,form,tiles,marches", [
+    (REAL, "step", (128, 192, 240, 256), (96, 176, 288, 352)),
+    (COMPLEX, "step", (128, 256), (96, 160, 240, 288)),
+    (COLOR, "step", (112, 128, 192, 224, 256), (72, 96, 144, 160, 288)),
+    (REAL, "masked_step", (160, 192, 256, 352), (128, 144, 288)),
+    (COMPLEX, "masked_step", (128, 240, 256), (96, 192, 224, 288)),
+    (REAL, "comp_step", (240, 256), (128, 224, 288)),
+    (COMPLEX, "comp_step", (256,), (128, 192, 240, 288))])
+def test_a_lattice_takes_the_kernel_that_measured_faster(fake, level, form, tiles, marches):
+    """The fused kernel (its tile lies in shared memory) against the marching one."""
+    for n in tiles + marches:
+        getattr(Lattice(level, n), form)()
+        assert (fake.fake_dynamic_smem() > 0) == (n in tiles), n
