@@ -28,6 +28,7 @@
 #include <cmath>
 #include <cstdio>
 #include <mutex>
+#include <type_traits>
 
 #include "lfm_b200.h"
 #include "lfm_kernels.h"
@@ -78,8 +79,10 @@ __device__ __forceinline__ void load_cells(const float* p, float (&x)[V]) {
 }
 
 // A thread's column is V cells wide along k.  qmax: largest 4 dist^2 of an interior
-// cell (dist <= radius in float64).
-template <int LEVEL, int V>
+// cell (dist <= radius in float64).  PREV: all previous fields are given; a field without
+// one adds no kinetic energy, also where it is not finite (v - v is NaN there).  The test
+// in the march costs COMPLEX 256^3 25 us, so it is left out where it is not needed.
+template <int LEVEL, int V, bool PREV>
 __global__ void __launch_bounds__(kThreads, V == 4 ? 2 : (LEVEL == LFM_COLOR ? 2 : 4))
     metrics_partial_kernel(MetricsArgs a, int64_t qmax, int planes, int64_t items,
                            double* partials) {
@@ -133,8 +136,8 @@ __global__ void __launch_bounds__(kThreads, V == 4 ? 2 : (LEVEL == LFM_COLOR ? 2
 #pragma unroll
         for (int e = 0; e < V; ++e) {
           const double v = (double)c[q][e];
-          const double d = v - (double)o[e];  // 0 where no previous field is given
-          A.s[kKinetic] = fma(d, d, A.s[kKinetic]);
+          const double d = v - (double)o[e];
+          if (PREV || old) A.s[kKinetic] = fma(d, d, A.s[kKinetic]);
           const double di = (double)n[e] - (double)m[q][e];
           di2 = fma(di, di, di2);
           const double dj = (double)hi[e] - (double)lo[e];
@@ -264,13 +267,20 @@ cudaError_t launch_metrics(const MetricsArgs& a, double* partials, int rows, dou
     kernel<<<rows, kThreads, 0, stream>>>(a, qmax, planes, (n2 / V + kThreads - 1) / kThreads * chunks,
                                           partials);
   };
+  const bool prev = a.pr_prev && (a.level == LFM_REAL || a.pi_prev);
+  const auto run_level = [&](auto level) {
+    constexpr int L = decltype(level)::value;
+    if (wide)
+      prev ? run(metrics_partial_kernel<L, 4, true>, 4) : run(metrics_partial_kernel<L, 4, false>, 4);
+    else
+      prev ? run(metrics_partial_kernel<L, 1, true>, 1) : run(metrics_partial_kernel<L, 1, false>, 1);
+  };
   if (a.level == LFM_REAL)
-    wide ? run(metrics_partial_kernel<LFM_REAL, 4>, 4) : run(metrics_partial_kernel<LFM_REAL, 1>, 1);
+    run_level(std::integral_constant<int, LFM_REAL>{});
   else if (a.level == LFM_COMPLEX)
-    wide ? run(metrics_partial_kernel<LFM_COMPLEX, 4>, 4)
-         : run(metrics_partial_kernel<LFM_COMPLEX, 1>, 1);
+    run_level(std::integral_constant<int, LFM_COMPLEX>{});
   else
-    wide ? run(metrics_partial_kernel<LFM_COLOR, 4>, 4) : run(metrics_partial_kernel<LFM_COLOR, 1>, 1);
+    run_level(std::integral_constant<int, LFM_COLOR>{});
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   metrics_finish_kernel<<<1, 32 * kPartialStride, 0, stream>>>(partials, rows, out);

@@ -163,3 +163,26 @@ def test_metrics_at_the_edges_of_the_march(be, level, N, shift, with_prev):
     assert m["interior_cells"] == inner.size and m["nonfinite_cells"] == 0
     assert m["well_fraction"] == (inner < 17.0).mean()
     assert m["void_fraction"] == (inner > 18.0).mean()
+
+
+@pytest.mark.parametrize("level", [0, 1, 2])
+@pytest.mark.parametrize("N", [16, 17])
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_no_kinetic_energy_without_a_previous_field(be, level, N, bad):
+    """Also where Psi is not finite; at COMPLEX and COLOR with one of two previous fields
+    given, the other part's alone."""
+    from lfm_b200.metrics import device_metrics
+
+    rng = np.random.default_rng(N)
+    shape = ((3,) if level == 2 else ()) + (N, N, N)
+    pr, pi, pip = (rng.standard_normal(shape).astype(np.float32) for _ in range(3))
+    pr[..., 3, 4, 5] = bad
+    chi = dev(be, np.full((N, N, N), 19.0, np.float32))
+    im = dev(be, pi) if level else None
+    m = device_metrics(be.context.handle, level, N, dev(be, pr), None, im, None, chi, 0.02)
+    assert m["energy_kinetic"] == 0.0 and m["nonfinite_cells"] == 1
+    if level:
+        m = device_metrics(be.context.handle, level, N, dev(be, pr), None, im, dev(be, pip), chi,
+                           0.02)
+        want = 0.5 * (((pi.astype(np.float64) - pip) / 0.02) ** 2).sum()
+        assert m["energy_kinetic"] == pytest.approx(want, rel=ENERGY_RTOL)
