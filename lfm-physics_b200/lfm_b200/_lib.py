@@ -165,18 +165,23 @@ def set_step_path(path: int) -> None:
     call("lfm_set_step_path", int(path))
 
 
-def run_workspace(level: int, N: int, device):
-    """Zeroed workspace of lfm_leapfrog_run_f32 for one lattice; empty if the lattice does
-    not fit on chip or there is no memory for it (both take single steps)."""
+def run_workspace(level: int, N: int, device) -> tuple:
+    """Zeroed workspace of lfm_leapfrog_run_f32 for one lattice, and whether the lattice may
+    keep it; empty if the lattice does not fit on chip or there is no memory for it (both
+    take single steps).
+
+    One made under stream capture is zeroed by the graph's replays alone, so it is the
+    captured run's and not to be kept for others."""
     import torch
 
     n = ctypes.c_longlong(0)
     with torch.cuda.device(device):
         call("lfm_leapfrog_run_words", int(level), int(N), ctypes.byref(n))
+        keep = not torch.cuda.is_current_stream_capturing()
     try:
-        return torch.zeros(n.value, dtype=torch.int32, device=device)
+        return torch.zeros(n.value, dtype=torch.int32, device=device), keep
     except torch.OutOfMemoryError:
-        return torch.empty(0, dtype=torch.int32, device=device)
+        return torch.empty(0, dtype=torch.int32, device=device), keep
 
 
 def run_steps(name: str, *args) -> bool:

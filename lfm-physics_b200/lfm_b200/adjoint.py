@@ -111,16 +111,19 @@ class _Lattice:
         self.damp = True
 
     def _run(self, name: str, steps: int, fields, stores, damp: bool) -> bool:
-        if self.run_sync is None:
-            self.run_sync = _lib.run_workspace(int(self.level), self.N, self.device)
-        if self.run_sync.numel() == 0:
+        sync = self.run_sync
+        if sync is None:
+            sync, keep = _lib.run_workspace(int(self.level), self.N, self.device)
+            if keep:
+                self.run_sync = sync
+        if sync.numel() == 0:
             return False
         ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
         order = [ptr(t) for t in fields]
         tail = (self.table.data_ptr(), ctypes.byref(self.desc), int(damp), self.N, *self.common,
                 float(self.config.epsilon_w))
         where = (ptr(stores),)
-        end = (self.run_sync.data_ptr(), _stream_handle(self.device))
+        end = (sync.data_ptr(), _stream_handle(self.device))
         if name == "lfm_advance_run_f32":
             return _lib.run_steps(name, int(self.level), steps, *order, *where, *tail, *end)
         return _lib.run_steps(name, int(self.level), steps, *order, *tail, *where, *end)

@@ -354,19 +354,23 @@ class Evolver:
         if self._level == FieldLevel.COLOR:
             return False
         cfg = self.config
-        if self._run_sync is None:
-            self._run_sync = _lib.run_workspace(int(self._level), self.N, self.device)
-        if self._run_sync.numel() == 0:
+        sync = self._run_sync
+        if sync is None:
+            sync, keep = _lib.run_workspace(int(self._level), self.N, self.device)
+            if keep:
+                self._run_sync = sync
+        if sync.numel() == 0:
             return False
         cur, prv = self._cur, 1 - self._cur
         pi = ((self._pi[cur].data_ptr(), self._pi[prv].data_ptr()) if self._has_imag
               else (None, None))
         if not _lib.run_steps(
-                "lfm_leapfrog_run_f32", int(self._level), steps, self._pr[cur].data_ptr(), self._pr[prv].data_ptr(), *pi,
+                "lfm_leapfrog_run_f32", int(self._level), steps, self._pr[cur].data_ptr(),
+                self._pr[prv].data_ptr(), *pi,
                 self._chi[cur].data_ptr(), self._chi[prv].data_ptr(), self._table_dev.data_ptr(),
                 ctypes.byref(self._desc), 1 if self._damp else 0, self.N, float(self._dt2),
                 float(cfg.kappa), float(cfg.lambda_self), float(cfg.chi0), float(cfg.e0_sq),
-                float(cfg.epsilon_w), None, self._run_sync.data_ptr(),
+                float(cfg.epsilon_w), None, sync.data_ptr(),
                 _stream_handle(self.device)):
             return False
         if steps % 2:

@@ -221,3 +221,38 @@ def test_batch_keeps_single_steps_where_it_must(be):
         assert not small._run_on_chip(4)
     finally:
         _lib.set_step_path(_lib.PATH_AUTO)
+
+
+@pytest.mark.gpu
+def test_a_workspace_made_under_capture_is_not_kept(be):
+    """Its zeroes come with the graph's replays: runs outside the graph need their own."""
+    import torch
+
+    from lfm_b200 import adjoint
+
+    a, b = _evolver(COMPLEX, 32, 5, be), _evolver(COMPLEX, 32, 5, be)
+    b.use_graphs = False
+    a.evolve(3)
+    b.evolve(3)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        a.evolve(8)
+    a.step -= 8  # nothing has run yet
+    assert a._run_sync is None
+    for again in (lambda: a.evolve(8), g.replay, lambda: a.evolve(8), g.replay):
+        again()
+        b.evolve(8)
+        a.step = b.step
+        _same(a, b)
+    assert a._run_sync.numel() > 0
+    a.synchronize()
+
+    lat = adjoint._lattice_for(gravity_em(36, kappa=1.25 / 63.0), be)
+    state = [t.clone().reshape(36, 36, 36) for t in lat.state()]
+    g = torch.cuda.CUDAGraph()
+    with torch.no_grad():
+        with torch.cuda.graph(g):
+            adjoint.leapfrog(lat.config, state, 6, backend=be)
+        assert lat.run_sync is None
+        adjoint.leapfrog(lat.config, state, 6, backend=be)
+    assert lat.run_sync.numel() > 0
