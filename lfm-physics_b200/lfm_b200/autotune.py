@@ -111,17 +111,29 @@ def batch_signature(configs) -> str:
 
 
 def tune_batch(batch, candidates=None, steps: int = 6, use_cache: bool = True) -> dict:
-    """Pick the fastest tuning for `batch` and apply it; returns {"best", "trials"}."""
+    """Pick the fastest tuning for `batch` and apply it; returns {"best", "trials"}.
+
+    A full search (no candidates given) times the on-chip run too, where the lattices fit
+    ("on_chip_ms_per_step"): evolve() keeps it where it is the faster ("on_chip_is_faster"),
+    and the best tuning is then that of single steps alone."""
     key = f"{_device_name(batch.device)}|{batch_signature(batch.configs)}"
     if use_cache and candidates is None:
         hit = _load_cache().get(key)
-        if hit is not None:
+        if hit is not None and "on_chip_is_faster" in hit:  # (entries of before lack it)
             batch.retune(hit["best"])
+            batch._on_chip = hit["on_chip_is_faster"]
             return hit
     saved = batch._arena.clone()
     saved_state = (batch._cur, batch._damp, batch.step)
     trials = []
+    on_chip = None
     try:
+        if candidates is None:
+            batch.retune(None)
+            if batch._run_on_chip(2):
+                # ten times the steps: a run's launch and fill come once for all of them
+                on_chip = 0.1 * _time_ms(batch.device,
+                                         lambda k: batch._run_on_chip(max(10 * k, 2)), steps)
         for cand in candidates or BATCH_CANDIDATES:
             try:
                 batch.retune(cand)
@@ -135,9 +147,12 @@ def tune_batch(batch, candidates=None, steps: int = 6, use_cache: bool = True) -
     if not trials:
         raise RuntimeError("no batch tuning candidate could be launched")
     best = min(trials, key=lambda t: t["ms_per_step"])
-    batch.retune(best["tuning"])
     out = {"best": best["tuning"], "ms_per_step": best["ms_per_step"], "trials": trials}
+    batch.retune(best["tuning"])
     if candidates is None:
+        out["on_chip_ms_per_step"] = on_chip
+        out["on_chip_is_faster"] = on_chip is not None and on_chip <= best["ms_per_step"]
+        batch._on_chip = out["on_chip_is_faster"]
         _store(key, out)
     return out
 

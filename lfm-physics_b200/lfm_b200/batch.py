@@ -112,8 +112,6 @@ class BatchedLattices:
         self._damp = False
         self._graphs: dict = {}
         self.tune_report = None
-        # a tuning of the tile kernel given by the caller asks for that kernel
-        self._on_chip = tuning is None or tuning == "auto"
         if tuning == "auto":
             from .autotune import tune_batch
 
@@ -124,8 +122,9 @@ class BatchedLattices:
 
     def retune(self, tuning: dict | None) -> None:
         """Re-plan the work list with another tuning (keys of lfm_batch_tuning:
-        threads, stages, item_cells, ctas_per_sm; missing or 0 = default).
-        The fields are untouched; captured graphs are dropped."""
+        threads, stages, item_cells, ctas_per_sm; missing or 0 = default).  A tuning of
+        the tile kernel asks for that kernel: evolve() holds the lattices on chip only
+        under None.  The fields are untouched; captured graphs are dropped."""
         t = _lib.BatchTuning()
         for k, v in (tuning or {}).items():
             setattr(t, k, int(v))
@@ -136,6 +135,7 @@ class BatchedLattices:
         if self._handle:
             _lib.load().lfm_batch_destroy(self._handle)
         self._handle = h
+        self._on_chip = tuning is None
         self._tuning = {f: getattr(t, f) for f, _ in t._fields_}
 
     def __len__(self) -> int:

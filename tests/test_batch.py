@@ -355,3 +355,53 @@ def test_autotune_lattice_pins_a_tile(be, tmp_path, monkeypatch):
         assert bits_equal(ev.get_chi(), ref.get_chi())
     finally:
         _lib.tune_set(0, 32, 0, 0, 0, 0)
+
+
+@pytest.mark.gpu
+def test_retune_decides_which_kernel_evolve_runs(be, monkeypatch):
+    """A tuning asks for the tile kernel, whether given at the start or later; None goes
+    back to the on-chip runs."""
+    from lfm_b200 import _lib
+
+    runs = []
+    run_steps = _lib.run_steps
+    monkeypatch.setattr(_lib, "run_steps", lambda *a: runs.append(a[0]) or run_steps(*a))
+    B, evs = run_pair(be, mixed_configs([16, 24]), 5)
+    assert "lfm_batch_run" in runs
+    for tuning in (dict(threads=128), None, dict(item_cells=2048)):
+        B.retune(tuning)
+        runs.clear()
+        B.evolve(6)
+        assert ("lfm_batch_run" in runs) == (tuning is None)
+        for ev in evs:
+            ev.evolve(6)
+        assert_same(B, evs)
+
+
+@pytest.mark.gpu
+def test_a_full_search_weighs_the_on_chip_run(be, tmp_path, monkeypatch):
+    """tuning="auto" keeps evolve() on chip where that is the faster, from the search as
+    from its cache; an entry that says nothing of it is searched again."""
+    import json
+
+    from lfm_b200 import autotune
+    from lfm_b200.batch import BatchedLattices
+
+    cache = tmp_path / "tune.json"
+    monkeypatch.setenv("LFM_B200_TUNE_CACHE", str(cache))
+    cands = [dict(threads=128), dict(threads=256)]
+    monkeypatch.setattr(autotune, "BATCH_CANDIDATES", cands)
+    cfgs = mixed_configs([16, 24])
+    rep = BatchedLattices(cfgs, backend=be, tuning="auto").tune_report
+    assert rep["on_chip_is_faster"] == (rep["on_chip_ms_per_step"] <= rep["ms_per_step"])
+    (key, entry), = json.loads(cache.read_text()).items()
+    for faster in (True, False):
+        cache.write_text(json.dumps({key: dict(entry, on_chip_is_faster=faster)}))
+        B = BatchedLattices(cfgs, backend=be, tuning="auto")
+        assert B._on_chip is faster and B._tuning["threads"] == entry["best"]["threads"]
+    old = {k: v for k, v in entry.items() if not k.startswith("on_chip")}
+    cache.write_text(json.dumps({key: old}))
+    rep = BatchedLattices(cfgs, backend=be, tuning="auto").tune_report
+    assert "on_chip_is_faster" in rep and len(rep["trials"]) == 2
+    big = BatchedLattices(mixed_configs([112, 16]), backend=be, tuning="auto")
+    assert big.tune_report["on_chip_ms_per_step"] is None and big._on_chip is False
