@@ -417,8 +417,9 @@ typedef struct lfm_batch lfm_batch;
 /* `steps` steps of every lattice with the state held on chip, waves of lattices one
  * after another (the same bits as `steps` calls of lfm_batch_step; the current fields
  * are then in slot parity + steps mod 2).  LFM_ERR_UNSUPPORTED, with nothing launched,
- * when a lattice does not fit on chip or a wave has no room there, steps < 2 or a step
- * path is forced. */
+ * when a lattice does not fit on chip or a wave has no room there, steps < 2, a step path
+ * is forced, or the first run of a batch made with a tuning comes under stream capture
+ * (its waves are planned then, and memory for them allocated). */
 int lfm_batch_run(lfm_batch* batch, int steps, int parity, int damp_prev, void* stream);
 
 

@@ -1519,7 +1519,7 @@ int plan_batch(const lfm_lattice_desc* L, int count, const lfm_batch_tuning& t, 
 }  // namespace
 
 struct lfm_batch {
-  int device = 0;
+  int device = 0, sms = 0;
   int stages = 3;
   int tab_off = -1;
   lfm::BatchLattice* d_lat = nullptr;
@@ -1529,9 +1529,42 @@ struct lfm_batch {
   int class_off[lfm::kBatchClasses] = {}, class_n[lfm::kBatchClasses] = {};
   // on-chip runs (lfm_batch_run): the lattices, their waves and the waves' workspace
   std::vector<lfm::BatchLattice> lat;
+  bool planned = false;
   std::vector<lfm::ResidentWavePlan> waves;
   uint32_t* d_sync = nullptr;
 };
+
+namespace {
+
+// The batch's waves of lattices held on chip and their workspace; none where a lattice
+// does not fit or there is no memory for it (the lattices take single steps).
+void plan_waves(lfm_batch* B) {
+  B->planned = true;
+  const int count = (int)B->lat.size();
+  std::vector<int> level(count), edge(count);
+  for (int l = 0; l < count; ++l) {
+    level[l] = B->lat[l].level;
+    edge[l] = B->lat[l].N;
+  }
+  if (!lfm::resident_waves(level.data(), edge.data(), count, B->sms, &B->waves)) return;
+  long long words = 0;
+  for (const lfm::ResidentWavePlan& w : B->waves) {
+    long long sum = 0;
+    for (const lfm::ResidentPlan& p : w.plans) sum += p.words;
+    words = std::max(words, sum);
+  }
+  cudaError_t e = cudaMalloc(&B->d_sync, 4 * (size_t)words);
+  if (e == cudaSuccess) e = cudaMemset(B->d_sync, 0, 4 * (size_t)words);
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    if (B->d_sync) cudaFree(B->d_sync);
+    B->d_sync = nullptr;
+    B->waves.clear();
+  }
+}
+
+}  // namespace
 
 extern "C" {
 
@@ -1623,6 +1656,7 @@ int lfm_batch_create(const lfm_lattice_desc* lattices, int count,
   }
   lfm_batch* B = new lfm_batch;
   B->device = device;
+  B->sms = sms;
   B->stages = t.stages;
   B->tab_off = plan.tab_off;
   B->nitems = (int)plan.items.size();
@@ -1650,31 +1684,12 @@ int lfm_batch_create(const lfm_lattice_desc* lattices, int count,
     lfm_batch_destroy(B);
     return cuda_fail(e, "batch descriptors");
   }
-  // Waves of lattices held on chip, for lfm_batch_run.
-  std::vector<int> level(count), edge(count);
-  for (int l = 0; l < count; ++l) {
-    level[l] = dev[l].level;
-    edge[l] = dev[l].N;
-  }
-  double cycles = 0.0;
-  if (lfm::resident_waves(level.data(), edge.data(), count, sms, &B->waves, &cycles)) {
-    long long words = 0;
-    for (const lfm::ResidentWavePlan& w : B->waves) {
-      long long sum = 0;
-      for (const lfm::ResidentPlan& p : w.plans) sum += p.words;
-      words = std::max(words, sum);
-    }
-    e = cudaMalloc(&B->d_sync, 4 * (size_t)words);
-    if (e == cudaSuccess) e = cudaMemset(B->d_sync, 0, 4 * (size_t)words);
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    if (e != cudaSuccess) {  // no memory for it: the lattices take single steps
-      cudaGetLastError();
-      if (B->d_sync) cudaFree(B->d_sync);
-      B->d_sync = nullptr;
-      B->waves.clear();
-    }
-  }
   B->lat = std::move(dev);
+  // A tuning asks for the tile kernel: waves are planned (0.8 ms) if a run comes all the
+  // same.
+  if (!tuning || (!tuning->threads && !tuning->stages && !tuning->item_cells &&
+                  !tuning->ctas_per_sm))
+    plan_waves(B);
   *out = B;
   return LFM_OK;
 }
@@ -1682,6 +1697,8 @@ int lfm_batch_create(const lfm_lattice_desc* lattices, int count,
 int lfm_batch_run(lfm_batch* batch, int steps, int parity, int damp_prev, void* stream) {
   if (!batch) return fail(LFM_ERR_INVALID_ARG, "null batch");
   if (parity != 0 && parity != 1) return fail(LFM_ERR_INVALID_ARG, "parity %d", parity);
+  if (steps >= 2 && !batch->planned && !capturing(static_cast<cudaStream_t>(stream)))
+    plan_waves(batch);
   if (batch->waves.empty() || steps < 2)
     return fail(LFM_ERR_UNSUPPORTED, "batch run: %d steps, %zu waves", steps, batch->waves.size());
   if (g_path.load() != 0) return fail(LFM_ERR_UNSUPPORTED, "batch run: a step path is forced");

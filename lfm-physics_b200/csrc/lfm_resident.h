@@ -59,9 +59,9 @@ struct ResidentWavePlan {
 constexpr int kWaveLattices = 32;  // at most, in a wave
 
 // The waves that run `count` lattices on chip one wave after another, those of the most
-// blocks first, and the model's cycles of a step through all of them; false if a lattice does not fit or its N is odd.
+// blocks first; false if a lattice does not fit or its N is odd.
 bool resident_waves(const int* level, const int* N, int count, int sms,
-                    std::vector<ResidentWavePlan>* waves, double* cycles);
+                    std::vector<ResidentWavePlan>* waves);
 
 // One wave: the same steps, sync and status for all; packets apart.
 cudaError_t launch_resident_wave(const ResidentArgs* a, int count, cudaStream_t stream);

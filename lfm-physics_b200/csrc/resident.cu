@@ -703,7 +703,7 @@ bool resident_plan(int level, int N, int sms, ResidentPlan* out) {
 // the fewest blocks that make a step in T (or as fast as it can), the largest go
 // first into the first wave with room, and what a wave has left speeds its slowest
 // lattice up.  The T of the smallest total is taken.
-static double pack_level(const int* N, const std::vector<int>& idx, int level, int sms,
+static void pack_level(const int* N, const std::vector<int>& idx, int level, int sms,
                          std::vector<ResidentWavePlan>* out) {
   double best_total = 1e300;
   std::vector<ResidentWavePlan> best;
@@ -752,13 +752,11 @@ static double pack_level(const int* N, const std::vector<int>& idx, int level, i
     }
   }
   out->insert(out->end(), best.begin(), best.end());
-  return best_total;
 }
 
 bool resident_waves(const int* level, const int* N, int count, int sms,
-                    std::vector<ResidentWavePlan>* waves, double* cycles) {
+                    std::vector<ResidentWavePlan>* waves) {
   sms = std::min(sms, kMaxBlocks);
-  *cycles = 0.0;
   waves->clear();
   for (int lv : {LFM_REAL, LFM_COMPLEX}) {
     std::vector<int> idx;
@@ -767,7 +765,7 @@ bool resident_waves(const int* level, const int* N, int count, int sms,
       if (!resident_plan(level[l], N[l], sms, &p) || N[l] % 2) return false;
       if (level[l] == lv) idx.push_back(l);
     }
-    if (!idx.empty()) *cycles += pack_level(N, idx, lv, sms, waves);
+    if (!idx.empty()) pack_level(N, idx, lv, sms, waves);
   }
   // the most blocks first, so that a launch the device has no room for is the first one
   std::stable_sort(waves->begin(), waves->end(),

@@ -12,7 +12,9 @@
 
 namespace {
 constexpr int kSms = 148, kOptin = 227 * 1024, kDefault = 48 * 1024;
-int device = 0, free_sms = kSms, launches = 0, refusals = 0, shared = 0;
+int device = 0, free_sms = kSms, launches = 0, refusals = 0, shared = 0,
+    allocations = 0;
+bool capturing = false;
 cudaError_t last = cudaSuccess;
 std::map<std::pair<int, const void*>, int> limit;  // raised limits: (device, kernel)
 struct Config {
@@ -39,6 +41,8 @@ cudaError_t launch(const void* kernel, dim3 grid, size_t smem, bool cooperative)
 
 extern "C" {
 int fake_launches() { return launches; }
+int fake_allocations() { return allocations; }
+void fake_capture(int on) { capturing = on; }
 int fake_refusals() { return refusals; }
 int fake_dynamic_smem() { return shared; }  // of the last launch
 int fake_last_error() { return last; }
@@ -46,6 +50,7 @@ void fake_free_sms(int n) { free_sms = n; }
 void fake_reset() {
   device = launches = refusals = 0;
   free_sms = kSms;
+  capturing = false;
   last = cudaSuccess;
 }
 
@@ -58,10 +63,14 @@ cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
 cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* s) {
-  *s = cudaStreamCaptureStatusNone;
+  *s = capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
   return cudaSuccess;
 }
-cudaError_t cudaMalloc(void** p, size_t n) { *p = calloc(1, n); return cudaSuccess; }
+cudaError_t cudaMalloc(void** p, size_t n) {
+  ++allocations;
+  *p = calloc(1, n);
+  return cudaSuccess;
+}
 cudaError_t cudaFree(void* p) { free(p); return cudaSuccess; }
 cudaError_t cudaMemset(void* p, int v, size_t n) { memset(p, v, n); return cudaSuccess; }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {

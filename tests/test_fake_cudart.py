@@ -104,10 +104,10 @@ class Lattice:
         return d
 
 
-def batch(lattices):
+def batch(lattices, **tuning):
     descs = (_lib.LatticeDesc * len(lattices))(*[x.desc() for x in lattices])
-    h = ctypes.c_void_p()
-    _lib.call("lfm_batch_create", descs, len(lattices), None, ctypes.byref(h))
+    h, t = ctypes.c_void_p(), _lib.BatchTuning(**tuning)
+    _lib.call("lfm_batch_create", descs, len(lattices), ctypes.byref(t), ctypes.byref(h))
     return h
 
 
@@ -173,3 +173,20 @@ def test_a_lattice_takes_the_kernel_that_measured_faster(fake, level, form, tile
     for n in tiles + marches:
         getattr(Lattice(level, n), form)()
         assert (fake.fake_dynamic_smem() > 0) == (n in tiles), n
+
+
+def test_a_tuned_batch_plans_its_waves_when_a_run_comes(fake):
+    """retune() and a tuning search make batches that step with the tile kernel."""
+    lats = [Lattice(REAL, 32), Lattice(COMPLEX, 16)]
+    start = fake.fake_allocations()
+    plain = batch(lats)
+    with_waves = fake.fake_allocations() - start
+    tuned = batch(lats, threads=128)
+    assert fake.fake_allocations() - start == 2 * with_waves - 1
+    _lib.call("lfm_batch_step", tuned, 0, 0, None)
+    fake.fake_capture(1)
+    assert _lib.run_steps("lfm_batch_run", plain, 4, 0, 0, None) is True
+    assert _lib.run_steps("lfm_batch_run", tuned, 4, 0, 0, None) is False
+    fake.fake_capture(0)
+    assert _lib.run_steps("lfm_batch_run", tuned, 4, 0, 0, None) is True
+    assert fake.fake_allocations() - start == 2 * with_waves
