@@ -177,9 +177,9 @@ def tune_lattice(evolver, candidates=None, steps: int = 20, use_cache: bool = Tr
     key = f"{_device_name(evolver.device)}|lattice:{level}:{N}"
     if use_cache and candidates is None:
         hit = _load_cache().get(key)
-        if hit is not None:
+        if hit is not None and "untuned_is_faster" in hit:  # (entries of before lack it)
             b = hit["best"]
-            if not hit.get("untuned_is_faster"):
+            if not hit["untuned_is_faster"]:
                 _lib.tune_set(level, N, b["tj"], b["stages"], b["ic"], b["vec"])
             return hit
     if evolver._mode != "resident":

@@ -405,3 +405,33 @@ def test_a_full_search_weighs_the_on_chip_run(be, tmp_path, monkeypatch):
     assert "on_chip_is_faster" in rep and len(rep["trials"]) == 2
     big = BatchedLattices(mixed_configs([112, 16]), backend=be, tuning="auto")
     assert big.tune_report["on_chip_ms_per_step"] is None and big._on_chip is False
+
+
+@pytest.mark.gpu
+def test_a_lattice_cache_entry_without_the_untuned_time_is_searched_again(be, tmp_path,
+                                                                          monkeypatch):
+    """A pinned tile shuts the on-chip run and the marching kernel off: an entry that does
+    not say whether it is faster than they are pins nothing."""
+    import json
+
+    from lfm_b200 import Evolver, _lib, autotune
+    from lfm_b200.config import gravity_only
+
+    cache = tmp_path / "tune.json"
+    monkeypatch.setenv("LFM_B200_TUNE_CACHE", str(cache))
+    monkeypatch.setattr(autotune, "lattice_candidates",
+                        lambda level: [dict(vec=4, tj=8, stages=3, ic=0)])
+    ev = Evolver(gravity_only(32), backend=be)
+    try:
+        rep = autotune.tune_lattice(ev, steps=4)
+        assert rep["untuned_is_faster"] and ev._run_on_chip(2)  # one launch against four
+        (key, entry), = json.loads(cache.read_text()).items()
+        old = {k: v for k, v in entry.items() if not k.startswith("untuned")}
+        cache.write_text(json.dumps({key: old}))
+        rep = autotune.tune_lattice(ev, steps=4)
+        assert "untuned_is_faster" in rep and ev._run_on_chip(2)
+        cache.write_text(json.dumps({key: dict(entry, untuned_is_faster=False)}))
+        autotune.tune_lattice(ev, steps=4)
+        assert not ev._run_on_chip(2)  # pinned
+    finally:
+        _lib.tune_set(0, 32, 0, 0)
