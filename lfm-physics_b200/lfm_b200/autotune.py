@@ -191,12 +191,13 @@ def tune_lattice(evolver, candidates=None, steps: int = 20, use_cache: bool = Tr
     prev_path = None
     trials = []
     untuned = None
-    if candidates is None:  # the kernel that runs without a tile (on chip, or marching)
-        _lib.tune_set(level, N, 0, 0)
-        evolver.evolve(4)
-        untuned = _time_ms(evolver.device, evolver.evolve, max(steps, 4))
-    _lib.set_step_path(_lib.PATH_FUSED)
     try:
+        if candidates is None:  # the kernel that runs without a tile (on chip, or marching)
+            _lib.tune_set(level, N, 0, 0)
+            evolver._graphs = {}  # of a tile that was pinned
+            evolver.evolve(4)
+            untuned = _time_ms(evolver.device, evolver.evolve, max(steps, 4))
+        _lib.set_step_path(_lib.PATH_FUSED)
         for cand in candidates or lattice_candidates(level):
             _lib.tune_set(level, N, cand["tj"], cand["stages"], cand["ic"], cand["vec"])
             evolver._graphs = {}

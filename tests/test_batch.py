@@ -435,3 +435,42 @@ def test_a_lattice_cache_entry_without_the_untuned_time_is_searched_again(be, tm
         assert not ev._run_on_chip(2)  # pinned
     finally:
         _lib.tune_set(0, 32, 0, 0)
+
+
+@pytest.mark.gpu
+def test_the_untuned_time_is_that_of_the_untuned_kernel(be, tmp_path, monkeypatch):
+    """Graphs captured under a pinned tile are not replayed for it, and a failure while it
+    is taken leaves the lattice as it was."""
+    import torch
+
+    from lfm_b200 import Evolver, _lib, autotune
+    from lfm_b200.config import gravity_only
+
+    N = 112
+    monkeypatch.setenv("LFM_B200_TUNE_CACHE", str(tmp_path / "tune.json"))
+    tile = dict(vec=4, tj=8, stages=3, ic=0)
+    monkeypatch.setattr(autotune, "lattice_candidates", lambda level: [tile])
+    ev = Evolver(gravity_only(N), backend=be)
+    time_ms = autotune._time_ms
+    try:
+        _lib.tune_set(0, N, tile["tj"], tile["stages"], 0, tile["vec"])
+        ev.evolve(8)
+        pinned = list(ev._graphs.values())
+        before = {k: v.clone() for k, v in ev.device_state().items()}
+
+        def check(device, fn, steps):
+            fn(steps)
+            assert not any(g is p for g in ev._graphs.values() for p in pinned)
+            raise RuntimeError("planted")
+
+        monkeypatch.setattr(autotune, "_time_ms", check)
+        with pytest.raises(RuntimeError, match="planted"):
+            autotune.tune_lattice(ev, steps=4)
+        assert ev.step == 8
+        assert all(torch.equal(v, before[k]) for k, v in ev.device_state().items())
+        monkeypatch.setattr(autotune, "_time_ms", time_ms)
+        rep = autotune.tune_lattice(ev, steps=4)
+        assert ev.step == 8 and rep["untuned_ms_per_step"] > 0
+        assert all(torch.equal(v, before[k]) for k, v in ev.device_state().items())
+    finally:
+        _lib.tune_set(0, N, 0, 0)
