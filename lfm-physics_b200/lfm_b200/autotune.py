@@ -196,7 +196,9 @@ def tune_lattice(evolver, candidates=None, steps: int = 20, use_cache: bool = Tr
             _lib.tune_set(level, N, 0, 0)
             evolver._graphs = {}  # of a tile that was pinned
             evolver.evolve(4)
-            untuned = _time_ms(evolver.device, evolver.evolve, max(steps, 4))
+            # ten times the steps: the tiles are timed as graphs, without the host's part
+            untuned = 0.1 * _time_ms(evolver.device, lambda k: evolver.evolve(10 * k),
+                                     max(steps, 4))
         _lib.set_step_path(_lib.PATH_FUSED)
         for cand in candidates or lattice_candidates(level):
             _lib.tune_set(level, N, cand["tj"], cand["stages"], cand["ic"], cand["vec"])

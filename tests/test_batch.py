@@ -424,12 +424,12 @@ def test_a_lattice_cache_entry_without_the_untuned_time_is_searched_again(be, tm
     ev = Evolver(gravity_only(32), backend=be)
     try:
         rep = autotune.tune_lattice(ev, steps=4)
-        assert rep["untuned_is_faster"] and ev._run_on_chip(2)  # one launch against four
+        assert ev._run_on_chip(2) == rep["untuned_is_faster"]
         (key, entry), = json.loads(cache.read_text()).items()
         old = {k: v for k, v in entry.items() if not k.startswith("untuned")}
         cache.write_text(json.dumps({key: old}))
         rep = autotune.tune_lattice(ev, steps=4)
-        assert "untuned_is_faster" in rep and ev._run_on_chip(2)
+        assert ev._run_on_chip(2) == rep["untuned_is_faster"]
         cache.write_text(json.dumps({key: dict(entry, untuned_is_faster=False)}))
         autotune.tune_lattice(ev, steps=4)
         assert not ev._run_on_chip(2)  # pinned
@@ -474,3 +474,26 @@ def test_the_untuned_time_is_that_of_the_untuned_kernel(be, tmp_path, monkeypatc
         assert all(torch.equal(v, before[k]) for k, v in ev.device_state().items())
     finally:
         _lib.tune_set(0, N, 0, 0)
+
+
+@pytest.mark.gpu
+def test_the_untuned_time_leaves_out_the_hosts_part(be, tmp_path, monkeypatch):
+    """As the tiles' does: at 32^3 four on-chip steps take 8 us, their launch from Python
+    twice that, four steps of the tile 27."""
+    from lfm_b200 import Evolver, _lib, autotune
+    from lfm_b200.config import gravity_only
+
+    monkeypatch.setenv("LFM_B200_TUNE_CACHE", str(tmp_path / "tune.json"))
+    monkeypatch.setattr(autotune, "lattice_candidates",
+                        lambda level: [dict(vec=4, tj=8, stages=3, ic=0)])
+    ev = Evolver(gravity_only(32), backend=be)
+    asked = []
+    time_ms = autotune._time_ms
+    monkeypatch.setattr(autotune, "_time_ms", lambda dev, fn, steps: time_ms(
+        dev, lambda k: asked.append(ev.step) or fn(k), steps))
+    try:
+        autotune.tune_lattice(ev, steps=4)
+        first, second = asked
+        assert second - first >= 10  # the warm-up: ten steps for the one asked for
+    finally:
+        _lib.tune_set(0, 32, 0, 0)
