@@ -160,9 +160,30 @@ def call(name: str, *args) -> None:
     check(getattr(load(), name)(*args), name)
 
 
+_path = PATH_AUTO
+_tiles: set = set()
+
+
 def set_step_path(path: int) -> None:
     """Choose the step kernel: 0 automatic, 1 direct, 2 fused 2.5D only."""
+    global _path
     call("lfm_set_step_path", int(path))
+    _path = int(path)
+
+
+def step_forced(level=None, N=None) -> bool:
+    """Whether a step path is forced (set_step_path), or a tile for (level, N) (tune_set)."""
+    return _path != PATH_AUTO or (level is not None and (int(level), int(N)) in _tiles)
+
+
+def run_words(level: int, N: int, device) -> int:
+    """Words of a run's workspace (lfm_leapfrog_run_words): 0 if the lattice does not fit."""
+    import torch
+
+    n = ctypes.c_longlong(0)
+    with torch.cuda.device(device):
+        call("lfm_leapfrog_run_words", int(level), int(N), ctypes.byref(n))
+    return n.value
 
 
 def run_workspace(level: int, N: int, device) -> tuple:
@@ -174,12 +195,11 @@ def run_workspace(level: int, N: int, device) -> tuple:
     captured run's and not to be kept for others."""
     import torch
 
-    n = ctypes.c_longlong(0)
+    words = run_words(level, N, device)
     with torch.cuda.device(device):
-        call("lfm_leapfrog_run_words", int(level), int(N), ctypes.byref(n))
         keep = not torch.cuda.is_current_stream_capturing()
     try:
-        return torch.zeros(n.value, dtype=torch.int32, device=device), keep
+        return torch.zeros(words, dtype=torch.int32, device=device), keep
     except torch.OutOfMemoryError:
         return torch.empty(0, dtype=torch.int32, device=device), keep
 
@@ -198,6 +218,7 @@ def run_steps(name: str, *args) -> bool:
 def tune_set(level: int, N: int, tj: int, stages: int, ic: int = 0, vec: int = 0) -> None:
     """Force the fused kernel's tile configuration for (level, N); tj <= 0 clears it."""
     call("lfm_tune_set", int(level), int(N), int(vec), int(tj), int(stages), int(ic))
+    (_tiles.add if tj > 0 else _tiles.discard)((int(level), int(N)))
 
 
 def tune_get(level: int, N: int) -> dict | None:

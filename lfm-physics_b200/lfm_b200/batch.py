@@ -197,8 +197,11 @@ class BatchedLattices:
         return g
 
     def warm_graphs(self) -> None:
-        """Capture the step-block graphs now (nothing runs); needs one step done."""
-        if not self._damp:
+        """Capture the step-block graphs now (nothing runs); needs one step done.  A batch
+        that runs on chip replays none."""
+        if not self._damp or (self._on_chip and not _lib.step_forced() and all(
+                _lib.run_words(int(c.field_level), c.grid_size, self.device) > 0
+                for c in self.configs)):
             return
         saved = self._cur
         for c in (0, 1):

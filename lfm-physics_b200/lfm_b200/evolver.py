@@ -336,8 +336,13 @@ class Evolver:
 
     def warm_graphs(self) -> None:
         """Capture the two-step graphs of both slot parities now (nothing runs), so a
-        later evolve() does not capture inside a timed region.  Needs one step done."""
-        if self._mode != "resident" or not self._damp or (self._sa_on and not self._energy_ok):
+        later evolve() does not capture inside a timed region.  Needs one step done.
+        A lattice that runs on chip replays none: its workspace is made instead."""
+        if self._mode != "resident":
+            return
+        if not _lib.step_forced(self._level, self.N) and self._workspace().numel() > 0:
+            return
+        if not self._damp or (self._sa_on and not self._energy_ok):
             return
         saved = self._cur
         for c in (0, 1):
@@ -348,17 +353,23 @@ class Evolver:
     run_block = 4096
     """Most steps per launch of a lattice that fits on chip (bounds a launch's length)."""
 
+    def _workspace(self):
+        """The workspace of the on-chip runs; empty where the lattice takes single steps."""
+        if self._run_sync is not None:
+            return self._run_sync
+        sync, keep = _lib.run_workspace(int(self._level), self.N, self.device)
+        if keep:
+            self._run_sync = sync
+        return sync
+
     def _run_on_chip(self, steps: int) -> bool:
         """`steps` steps with the state held on chip (lfm_leapfrog_run_f32); False if the
         lattice does not fit, or a step path or tile is forced."""
-        if self._level == FieldLevel.COLOR:
+        if self._level == FieldLevel.COLOR or (
+                self._run_sync is None and _lib.step_forced(self._level, self.N)):
             return False
         cfg = self.config
-        sync = self._run_sync
-        if sync is None:
-            sync, keep = _lib.run_workspace(int(self._level), self.N, self.device)
-            if keep:
-                self._run_sync = sync
+        sync = self._workspace()
         if sync.numel() == 0:
             return False
         cur, prv = self._cur, 1 - self._cur

@@ -256,3 +256,34 @@ def test_a_workspace_made_under_capture_is_not_kept(be):
         assert lat.run_sync is None
         adjoint.leapfrog(lat.config, state, 6, backend=be)
     assert lat.run_sync.numel() > 0
+
+
+@pytest.mark.gpu
+def test_warm_graphs_captures_what_evolve_replays(be):
+    """Graphs for lattices that take single steps; for the others the workspace."""
+    import torch
+
+    from lfm_b200.batch import BatchedLattices
+
+    graphs = lambda ev: len(getattr(ev, "_graphs", {}))  # noqa: E731
+    for n, forced in ((32, False), (110, False), (32, True)):
+        ev = _evolver(REAL, n, 1, be)
+        ev.evolve(1)
+        if forced:
+            _lib.tune_set(REAL, n, 8, 3, 8, 4)
+        try:
+            ev.warm_graphs()
+            fits = n == 32 and not forced
+            assert graphs(ev) == (0 if fits else 2)
+            assert (ev._run_sync is not None and ev._run_sync.numel() > 0) == fits
+            before = torch.cuda.memory_stats(be.device)["allocation.all.allocated"]
+            ev.evolve(9)
+            assert torch.cuda.memory_stats(be.device)["allocation.all.allocated"] == before
+            assert graphs(ev) == (0 if fits else 2)
+        finally:
+            _lib.tune_set(REAL, n, 0, 0)
+    for tuning in (None, dict(threads=128)):
+        B = BatchedLattices([gravity_only(32), gravity_em(16)], backend=be, tuning=tuning)
+        B.evolve(1)
+        B.warm_graphs()
+        assert len(B._graphs) == (0 if tuning is None else 4)
