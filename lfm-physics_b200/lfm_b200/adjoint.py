@@ -128,24 +128,46 @@ class _Lattice:
             return _lib.run_steps(name, int(self.level), steps, *order, *where, *tail, *end)
         return _lib.run_steps(name, int(self.level), steps, *order, *tail, *where, *end)
 
-    def run(self, steps: int, stores=None) -> bool:
-        """`steps` steps in place with the state held on chip (lfm_leapfrog_run_f32), the
-        time levels listed in `stores` (store_table) stored on the way; False, with
-        nothing done, if the lattice has to take single steps."""
-        c, p = self.cur, 1 - self.cur
-        pi = (self.pi[c], self.pi[p]) if self.cx else (None, None)
-        if not self._run("lfm_leapfrog_run_f32", steps,
-                         (self.pr[c], self.pr[p], *pi, self.chi[c], self.chi[p]), stores,
-                         self.damp):
-            return False
-        self.cur = p if steps % 2 else c
-        self.damp = True
-        return True
+    run_block = 4096
+    """Most steps per on-chip launch (bounds a launch's length)."""
 
-    def advance_run(self, cur, prev, steps: int, stores, damp: bool) -> bool:
-        """The same out of place from (psi_r, psi_i, chi) triples (lfm_advance_run_f32)."""
-        return self._run("lfm_advance_run_f32", steps,
-                         (cur[0], prev[0], cur[1], prev[1], cur[2], prev[2]), stores, damp)
+    def _next_block(self, left: int) -> int:
+        """Steps of the next launch when `left` are to be done: no single one is left over
+        (a run takes two or more)."""
+        k = min(left, self.run_block)
+        return k - 1 if left - k == 1 else k
+
+    def run(self, steps: int, stores=None) -> int:
+        """`steps` steps in place with the state held on chip (lfm_leapfrog_run_f32), the
+        time levels listed in `stores` (store_table) stored on the way; how many were done:
+        none if the lattice has to take single steps."""
+        done = 0
+        while steps - done >= 2:
+            k = self._next_block(steps - done)
+            c, p = self.cur, 1 - self.cur
+            pi = (self.pi[c], self.pi[p]) if self.cx else (None, None)
+            if not self._run("lfm_leapfrog_run_f32", k,
+                             (self.pr[c], self.pr[p], *pi, self.chi[c], self.chi[p]),
+                             None if stores is None else stores[done:], self.damp):
+                break
+            self.cur = p if k % 2 else c
+            self.damp = True
+            done += k
+        return done
+
+    def advance_run(self, cur, prev, states, stores, damp: bool) -> int:
+        """The same out of place from (psi_r, psi_i, chi) triples to those in `states`, whose
+        addresses are in `stores` (lfm_advance_run_f32)."""
+        done = 0
+        while len(states) - done >= 2:
+            k = self._next_block(len(states) - done)
+            if not self._run("lfm_advance_run_f32", k,
+                             (cur[0], prev[0], cur[1], prev[1], cur[2], prev[2]),
+                             stores[done:], damp):
+                break
+            done += k
+            cur, prev, damp = states[done - 1], states[done - 2], True
+        return done
 
     def store_table(self, levels):
         """Device table of the buffers that the time levels of an on-chip run go to: one
@@ -316,10 +338,11 @@ class _Plan:
         lat = self.lat
         lat.cur, lat.damp = 0, False
         self._checkpoint(0)
-        if self.fwd_stores is not None and lat.run(self.steps, self.fwd_stores):
+        done = 0
+        if self.fwd_stores is not None:
+            done = lat.run(self.steps, self.fwd_stores)
             self.meta[1:] = [True] * (len(self.meta) - 1)
-            return
-        for t in range(self.steps):
+        for t in range(done, self.steps):
             if t and t % self.every == 0:
                 self._checkpoint(t // self.every)
             lat.step()
@@ -336,12 +359,12 @@ class _Plan:
             e0 = min(s0 + every, steps)
             c0, p0 = self.snaps[si]
             states = [c0] + self.seg[: e0 - s0]
-            if not (self.seg_stores is not None and e0 - s0 > 1
-                    and lat.advance_run(c0, p0, e0 - s0, self.seg_stores, self.meta[si])):
-                for t in range(s0, e0):
-                    u = t - s0
-                    lat.advance(states[u], p0 if u == 0 else states[u - 1], states[u + 1],
-                                self.meta[si] if u == 0 else True)
+            done = 0
+            if self.seg_stores is not None:
+                done = lat.advance_run(c0, p0, states[1:], self.seg_stores, self.meta[si])
+            for u in range(done, e0 - s0):
+                lat.advance(states[u], p0 if u == 0 else states[u - 1], states[u + 1],
+                            self.meta[si] if u == 0 else True)
             for t in range(e0 - 1, s0 - 1, -1):
                 # every step but the run's last (the first walked) takes its adjoints as
                 # the step before in the walk left them, all but its first leave them so
@@ -466,9 +489,8 @@ def leapfrog(config, state, steps: int, every: int | None = None, backend="auto"
         s is not None and s.requires_grad for s in state)
     if not needs_grad:
         lat.load(state)
-        if steps < 2 or not lat.run(steps):
-            for _ in range(steps):
-                lat.step()
+        for _ in range(lat.run(steps), steps):
+            lat.step()
         return tuple(None if o is None else o.reshape(lat.N, lat.N, lat.N) for o in lat.state())
     return LeapfrogFunction.apply(_plan_for(lat, steps, every), *state)
 

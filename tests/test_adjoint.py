@@ -414,3 +414,44 @@ def test_leapfrog_forward_matches_evolver(be):
     assert torch.equal(out[0].cpu(), torch.from_numpy(ev.get_psi_real()))
     assert torch.equal(out[4].cpu(), torch.from_numpy(ev.get_chi()))
     assert torch.equal(out[1].cpu(), torch.from_numpy(ev.get_psi_real_prev()))
+
+
+def _leapfrog(cfg, be, steps, every, *, single=False, run_block=None):
+    """Outputs and gradients of one leapfrog() on a fresh lattice, and the lengths of its
+    on-chip runs; single: without them."""
+    from lfm_b200 import adjoint
+
+    adjoint._LATTICES.clear()
+    lat = adjoint._lattice_for(cfg, be)
+    if single:
+        lat.run_sync = torch.empty(0, dtype=torch.int32, device=be.device)
+    if run_block:
+        lat.run_block = run_block
+    runs = []
+    run = lat._run
+    lat._run = lambda name, steps, *a: run(name, steps, *a) and (runs.append(steps) or True)
+    state = [None if t is None else t.float().requires_grad_(True)
+             for t in random_state(cfg.grid_size, lat.cx, be.device, 3)]
+    out = adjoint.leapfrog(cfg, state, steps, every=every, backend=be)
+    cot = [t.float() for t in random_state(cfg.grid_size, True, be.device, 4)]
+    loss = sum((o * c).sum() for o, c in zip(out, cot) if o is not None)
+    grads = torch.autograd.grad(loss, [t for t in state if t is not None])
+    with torch.no_grad():
+        plain = adjoint.leapfrog(cfg, state, steps, backend=be)
+    adjoint._LATTICES.clear()
+    return [t.detach().clone() for t in (*out, *grads, *plain) if t is not None], runs
+
+
+def _bits(a, b) -> bool:
+    return all(torch.equal(x.view(torch.int32), y.view(torch.int32)) for x, y in zip(a, b))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("level", ["real", "complex"])
+def test_on_chip_runs_of_leapfrog_have_a_length_limit(be, level):
+    cfg = config5_like(16, level == "complex")
+    want, runs = _leapfrog(cfg, be, 23, 8)
+    assert max(runs) == 23
+    for block in (2, 3, 5):
+        got, runs = _leapfrog(cfg, be, 23, 8, run_block=block)
+        assert runs and max(runs) <= block and _bits(want, got)
