@@ -455,3 +455,84 @@ def test_on_chip_runs_of_leapfrog_have_a_length_limit(be, level):
     for block in (2, 3, 5):
         got, runs = _leapfrog(cfg, be, 23, 8, run_block=block)
         assert runs and max(runs) <= block and _bits(want, got)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("level", ["real", "complex"])
+@pytest.mark.parametrize("N", [9, 21, 33, 35])
+def test_on_chip_segments_equal_single_steps_at_odd_edges(be, level, N):
+    """Checkpoints and segment states stored on the way; the last segment is one step."""
+    cfg = config5_like(N, level == "complex")
+    got, runs = _leapfrog(cfg, be, 13, 4)
+    assert set(runs) == {13, 4}  # (run once and captured once)
+    want, runs = _leapfrog(cfg, be, 13, 4, single=True)
+    assert not runs and _bits(got, want)
+
+
+def _clamped_steps(cfg, be, steps):
+    """A lattice and its states over `steps` steps, with cells that chi's clamp holds."""
+    from lfm_b200.adjoint import _Lattice
+
+    lat = _Lattice(cfg, be)
+    st = [None if t is None else t.float() for t in random_state(cfg.grid_size, lat.cx, be.device, 5)]
+    st[4][::5, ::3, 1::4] = -19.0  # with chi_prev = 19 the step goes to -57 and is clamped
+    flat = lambda t: None if t is None else t.reshape(-1).contiguous()  # noqa: E731
+    prev, cur = [flat(st[k]) for k in (1, 3, 5)], [flat(st[k]) for k in (0, 2, 4)]
+    states = [cur]
+    for t in range(steps):
+        out = lat.new_state_buffers()
+        lat.advance(states[-1], prev if t == 0 else states[-2], out, t > 0)
+        states.append(out)
+    return lat, states
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("level", ["real", "complex"])
+@pytest.mark.parametrize("N", [16, 21, 33, 35, 40])
+def test_a_chain_of_adjoint_steps_gives_the_single_steps_bits(be, level, N):
+    lat, states = _clamped_steps(config5_like(N, level == "complex"), be, 5)
+    assert (states[1][2] == -19.0).any()
+    results = []
+    for chained in (False, True):
+        g = [[None if t is None else t.float().reshape(-1).contiguous()
+              for t in random_state(N, lat.cx, be.device, 6)]]
+        g.append([None if t is None else torch.empty_like(t) for t in g[0]])
+        for t in range(4, -1, -1):
+            chain = ((1 if t < 4 else 0) | (2 if t > 0 else 0)) if chained else 0
+            lat.adjoint_step(states[t], states[t + 1], g[0], g[1], chain)
+            g.reverse()
+        results.append([t for t in g[0] if t is not None])
+    assert _bits(*results)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("level", ["real", "complex"])
+@pytest.mark.parametrize("N", [21, 33, 35, 44])
+def test_one_adjoint_step_at_odd_and_wide_edges_is_the_float64_vjp(be, level, N):
+    """Rows of an odd number of cells, and more than one tile along k: as at N = 16."""
+    from lfm_b200.adjoint import _Lattice
+    from lfm_b200.mask import boundary_mask
+
+    cx = level == "complex"
+    cfg = config5_like(N, cx)
+    dev = be.device
+    st, cot = random_state(N, cx, dev, 1), random_state(N, cx, dev, 2)
+    mask = torch.from_numpy(boundary_mask(N, cfg.boundary_fraction).reshape(N, N, N)).to(
+        dev, torch.float64)
+    inp = [None if t is None else t.clone().requires_grad_(True) for t in st]
+    common = (mask, cfg.dt**2, cfg.kappa, cfg.lambda_self, cfg.chi0, cfg.e0_sq)
+    if cx:
+        out = TR.step_complex(*inp, *common, cfg.epsilon_w)
+    else:
+        o = TR.step_real(inp[0], inp[1], inp[4], inp[5], *common)
+        out = (o[0], o[1], None, None, o[2], o[3])
+    pairs = [(o, c) for o, c in zip(out, cot) if o is not None]
+    want = torch.autograd.grad([o for o, _ in pairs], [t for t in inp if t is not None],
+                               [c for _, c in pairs])
+    lat = _Lattice(cfg, be)
+    f32 = lambda t: None if t is None else t.detach().float().reshape(-1).contiguous()  # noqa: E731
+    g_out = [f32(c) for c in cot]
+    g_in = [None if c is None else torch.empty_like(c) for c in g_out]
+    lat.adjoint_step([f32(st[0]), f32(st[2]), f32(st[4])], [None, None, f32(out[4])], g_out, g_in)
+    for got, w in zip([g for g in g_in if g is not None], want):
+        assert rel(got, w) < 2e-6, rel(got, w)

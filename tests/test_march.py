@@ -151,3 +151,71 @@ def test_color_steps(be, N, shift):
 
     for a, b in zip(*_direct(run)):
         assert np.array_equal(a, b)
+
+
+def _three_steps(be, kind, level, N):
+    """Fields after three steps of an evolver (the first from undamped previous fields)."""
+    from lfm_b200 import Evolver, SplitChiEvolver
+    from lfm_b200.compensated import CompensatedEvolver
+
+    make = {"plain": Evolver, "split": SplitChiEvolver, "comp": CompensatedEvolver,
+            "ab": lambda cfg, backend: Evolver(cfg, backend=backend, buffers="ab")}[kind]
+    rng = np.random.default_rng(N)
+    pr, pi, chi = (rng.standard_normal((N, N, N), dtype=np.float32) for _ in range(3))
+    ev = make((gravity_em if level else gravity_only)(N), backend=be)
+    ev.use_graphs = False
+    ev.set_psi_real(0.5 * pr)
+    if level:
+        ev.set_psi_imag(0.5 * pi)
+    ev.set_chi(19.0 + np.float32(1e-2) * chi)
+    ev.evolve(3)
+    return [ev.get_psi_real(), ev.get_chi()] + ([ev.get_psi_imag()] if level else [])
+
+
+@pytest.mark.parametrize("kind", ["plain", "split", "comp", "ab"])
+@pytest.mark.parametrize("level", [REAL, COMPLEX])
+@pytest.mark.parametrize("N", [150, 163])
+def test_marches_of_more_planes_than_the_queue_holds(be, level, N, kind):
+    """Five planes a march and more (the queue's slots come round again), the last march of
+    a column shorter than the others."""
+    for a, b in zip(*_direct(lambda: _three_steps(be, kind, level, N))):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+@pytest.mark.parametrize("kind", ["plain", "split", "comp", "ab"])
+@pytest.mark.parametrize("level", [REAL, COMPLEX])
+@pytest.mark.parametrize("N", [24, 48, 160, 240])
+def test_run_time_tiles_at_every_size(be, level, N, kind):
+    """The fused kernel's run-time tiles, also where another kernel is the faster one and
+    they run only when asked for."""
+    if (N, level) == (24, REAL) and kind != "split":
+        pytest.skip("no tile: rows of six threads")
+    _lib.set_step_path(_lib.PATH_FUSED)
+    try:
+        tile = _three_steps(be, kind, level, N)
+    finally:
+        _lib.set_step_path(_lib.PATH_AUTO)
+    for other in _direct(lambda: _three_steps(be, kind, level, N)):
+        for a, b in zip(tile, other):
+            assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+@pytest.mark.parametrize("N", [112, 150, 192])
+def test_color_steps_on_every_kernel(be, N):
+    """COLOR with a streamed mask where the chosen kernel is a tile (112, 192) or marches
+    (150: four planes a march), against the direct kernel."""
+    rng = np.random.default_rng(N)
+    n = N**3
+    f = lambda k: be.from_numpy(rng.standard_normal(k * n, dtype=np.float32))  # noqa: E731
+    ins = [f(3) * 0.5 for _ in range(4)] + [19.0 + 0.1 * f(1) for _ in range(2)]
+    mask = be.from_numpy(rng.random(n, dtype=np.float32))
+
+    def run():
+        import torch
+
+        out = [torch.empty_like(a) for a in ins]
+        be.step_color(*ins, mask, *out, N, 4e-4, 1 / 63, 4 / 31, 19.0, 0.01, 0.1, 1 / 189, 2 / 17)
+        return [be.to_numpy(o).view(np.uint32) for o in out]
+
+    for a, b in zip(*_direct(run)):
+        assert np.array_equal(a, b)
