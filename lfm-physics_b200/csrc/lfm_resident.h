@@ -18,7 +18,8 @@ struct ResidentPlan {
   int nbi = 0, nbj = 0, NI = 0, NJ = 0;
   int V = 0, segs = 0, threads = 0;
   int RS = 0;    // floats of a shared-memory row
-  int smem = 0;  // bytes of dynamic shared memory
+  int smem = 0;  // bytes of dynamic shared memory, of a lattice run by itself
+  bool small = false;  // fields laid out for small lattices then
   long long words = 0;  // 32-bit words of the workspace: 4 counters, two exchange buffers
   double cycles = 0;    // the model's time of a step
 };

@@ -48,6 +48,7 @@ constexpr int kMaxBlocks = 148;  // one block an SM
 // 3.99 against 3.53 us a step, 96^3 8.1 against 7.5): their k neighbours meet in
 // four-way bank conflicts, and half the threads are left to hide latency.
 constexpr int kCells = 2;
+constexpr int kSmallEdge = 36;
 constexpr int kSmemBytes = 226 * 1024;  // 227 KB opt-in less the static part
 
 template <int LEVEL>
@@ -114,9 +115,11 @@ struct Block {
 
 // Floats of a field's rows, at most: two slots and the halo.  COMPLEX 96^3 in 12 x
 // 12 blocks takes 4 + 164 rows of 100 floats = 16404; REAL 108^3 4 + 202 rows of
-// 112 = 22628.
-template <int LEVEL>
-constexpr int kFieldFloats = LEVEL == LFM_REAL ? 22656 : 16448;
+// 112 = 22628.  SMALL: lattices of up to 36^3 (4 + 34 rows of 40 = 1364), whose blocks of
+// 192 threads or fewer leave an SM registers for another's, so that runs on several
+// streams share the chip (with 180 KB a block one waited for the other's whole launch).
+template <int LEVEL, bool SMALL>
+constexpr int kFieldFloats = SMALL ? 1376 : LEVEL == LFM_REAL ? 22656 : 16448;
 
 // A thread's cells: k0 .. k0+V-1 of row jr, planes [pa, pb).
 struct Cells {
@@ -227,13 +230,13 @@ __device__ __forceinline__ void store_row(float* p, const float (&x)[2], const B
   if (T.last) p[-T.k0 - 1] = EVEN ? x[1] : x[0];
 }
 
-template <int LEVEL, bool EVEN, int PA, int PB, int PC>
+template <int LEVEL, bool EVEN, bool SMALL, int PA, int PB, int PC>
 __device__ __forceinline__ void plane(const StepConsts& c, float* sm, const Block& B,
                                       const Cells& T, const Step& S,
                                       QPlane<kCells> (&Q)[kFields<LEVEL>][3], int ii,
                                       RowOff& centre, RowWalk& walk, int& mask_at,
                                       const Destinations& D) {
-  constexpr int NS = kFields<LEVEL>, FS = kFieldFloats<LEVEL>, V = kCells;
+  constexpr int NS = kFields<LEVEL>, FS = kFieldFloats<LEVEL, SMALL>, V = kCells;
   const RowOff nxt = ii + 1 < B.ni ? walk.next : halo_plane(B, T, true);
   step_rows(walk);
 #pragma unroll
@@ -310,12 +313,12 @@ __device__ __forceinline__ void plane(const StepConsts& c, float* sm, const Bloc
 // A thread takes the V cells of group kg of every rows_a_round-th row, the first
 // kBatch rows at once: their packets are polled before the CTA's barrier, behind
 // which every thread is done with the halo of the time before.
-template <int LEVEL, bool EVEN>
+template <int LEVEL, bool EVEN, bool SMALL>
 __device__ __forceinline__ bool receive(float* sm, const Block& B, const Cells& T,
                                         const ulonglong2* in, const int* halo_src, int HR,
                                         uint32_t t, int first, int rows_a_round) {
   constexpr int V = kCells, NS = kFields<LEVEL>, NP = kPackets<LEVEL, V>, kBatch = 4;
-  constexpr int FS = kFieldFloats<LEVEL>;
+  constexpr int FS = kFieldFloats<LEVEL, SMALL>;
   constexpr int LAST = NS * V - 3 * (NP - 1);  // values in a group's last packet
   bool ok = true, met = false;
   for (int q = first; q < HR || !met; q += kBatch * rows_a_round) {
@@ -421,7 +424,7 @@ struct Wave {
   ResidentArgs lattice[LATTICES];
 };
 
-template <int LEVEL, bool EVEN, int THREADS, int LATTICES>
+template <int LEVEL, bool EVEN, int THREADS, int LATTICES, bool SMALL>
 __global__ void __launch_bounds__(THREADS, 1)
     resident_kernel(const __grid_constant__ Wave<LATTICES> W) {
   constexpr int V = kCells, NS = kFields<LEVEL>;
@@ -448,7 +451,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   B.ni = (bi + 1) * A.N / L.nbi - B.i0;
   B.j0 = bj * A.N / L.nbj;
   B.nj = (bj + 1) * A.N / L.nbj - B.j0;
-  constexpr int FS = kFieldFloats<LEVEL>;
+  constexpr int FS = kFieldFloats<LEVEL, SMALL>;
   float* mask_rows = sm + NS * FS;
   int* halo_row = reinterpret_cast<int*>(mask_rows + L.NI * L.NJ * B.N4);  // HR entries
   int* own_row = halo_row + HR;                                // NI * NJ entries
@@ -567,16 +570,17 @@ __global__ void __launch_bounds__(THREADS, 1)
       for (int f = 0; f < NS; ++f) load_rows<V>(Q[f][1], sm + f * FS, centre);
       int ii = T.pa, mask_at = (T.pa * B.NJ + T.jr) * B.N4 + T.k0;
       while (true) {
-        plane<LEVEL, EVEN, 0, 1, 2>(A.c, sm, B, T, S, Q, ii, centre, walk, mask_at, s_dst);
+        plane<LEVEL, EVEN, SMALL, 0, 1, 2>(A.c, sm, B, T, S, Q, ii, centre, walk, mask_at, s_dst);
         if (++ii >= T.pb) break;
-        plane<LEVEL, EVEN, 1, 2, 0>(A.c, sm, B, T, S, Q, ii, centre, walk, mask_at, s_dst);
+        plane<LEVEL, EVEN, SMALL, 1, 2, 0>(A.c, sm, B, T, S, Q, ii, centre, walk, mask_at, s_dst);
         if (++ii >= T.pb) break;
-        plane<LEVEL, EVEN, 2, 0, 1>(A.c, sm, B, T, S, Q, ii, centre, walk, mask_at, s_dst);
+        plane<LEVEL, EVEN, SMALL, 2, 0, 1>(A.c, sm, B, T, S, Q, ii, centre, walk, mask_at, s_dst);
         if (++ii >= T.pb) break;
       }
     }
     if (s + 1 == A.steps) break;
-    if (!receive<LEVEL, EVEN>(sm, B, T, packets, halo_src, HR, S.t, first_row, rows_a_round)) {
+    if (!receive<LEVEL, EVEN, SMALL>(sm, B, T, packets, halo_src, HR, S.t, first_row,
+                                     rows_a_round)) {
       s_abort = 1;
       atomicOr(A.status, LFM_ERR_DEVICE_TIMEOUT);
     }
@@ -594,10 +598,10 @@ __global__ void __launch_bounds__(THREADS, 1)
   }
 }
 
-template <int LEVEL, bool EVEN, int THREADS, int LATTICES>
+template <int LEVEL, bool EVEN, int THREADS, int LATTICES, bool SMALL>
 cudaError_t launch(const Wave<LATTICES>& w, int threads, int smem, cudaStream_t stream) {
   static SmemGrant grant;
-  const auto kernel = resident_kernel<LEVEL, EVEN, THREADS, LATTICES>;
+  const auto kernel = resident_kernel<LEVEL, EVEN, THREADS, LATTICES, SMALL>;
   const cudaError_t e = grant.raise((const void*)kernel, smem);
   if (e != cudaSuccess) return e;
   void* args[] = {const_cast<Wave<LATTICES>*>(&w)};
@@ -605,19 +609,24 @@ cudaError_t launch(const Wave<LATTICES>& w, int threads, int smem, cudaStream_t 
                                      args, (size_t)smem, stream);
 }
 
-template <int LEVEL>
+template <int LEVEL, bool EVEN>
 cudaError_t launch_level(const ResidentArgs& a, cudaStream_t stream) {
   Wave<1> w{1, {0, a.plan.nbi * a.plan.nbj}, {a}};
   const int t = a.plan.threads, sm = a.plan.smem;
-  if constexpr (LEVEL == LFM_COMPLEX)
-    return a.N % 2 == 0 ? launch<LEVEL, true, kThreadsComplex>(w, t, sm, stream)
-                        : launch<LEVEL, false, kThreadsComplex>(w, t, sm, stream);
-  else if (a.N % 2 == 0)
-    return t <= 384 ? launch<LEVEL, true, 384>(w, t, sm, stream)
-                    : launch<LEVEL, true, 512>(w, t, sm, stream);
-  else
-    return t <= 384 ? launch<LEVEL, false, 384>(w, t, sm, stream)
-                    : launch<LEVEL, false, 512>(w, t, sm, stream);
+  static_assert(kThreadsComplex == 384, "one block size for COMPLEX and the smaller REAL blocks");
+  if (a.plan.small) return launch<LEVEL, EVEN, 384, 1, true>(w, t, sm, stream);
+  if constexpr (LEVEL == LFM_REAL)
+    if (t > 384) return launch<LEVEL, EVEN, 512, 1, false>(w, t, sm, stream);
+  return launch<LEVEL, EVEN, 384, 1, false>(w, t, sm, stream);
+}
+
+// Bytes of dynamic shared memory of a block: the fields, the sponge rows, the row tables.
+int smem_bytes(int level, int N, int NI, int NJ, bool small) {
+  const bool cx = level == LFM_COMPLEX;
+  const int field = small ? kFieldFloats<LFM_REAL, true>
+                          : cx ? kFieldFloats<LFM_COMPLEX, false> : kFieldFloats<LFM_REAL, false>;
+  const int N4 = (N + 3) / 4 * 4, halo = 2 * (NJ + 2) + 2 * NI;
+  return 4 * ((cx ? 3 : 2) * field + NI * NJ * N4 + 2 * halo + NI * NJ);
 }
 
 template <int LEVEL>
@@ -630,13 +639,14 @@ cudaError_t launch_wave(const ResidentArgs* a, int count, cudaStream_t stream) {
     w.lattice[l] = a[l];
     w.first[l + 1] = w.first[l] + a[l].plan.nbi * a[l].plan.nbj;
     threads = std::max(threads, a[l].plan.threads);
-    smem = std::max(smem, a[l].plan.smem);
+    smem = std::max(smem, smem_bytes(LEVEL, a[l].N, a[l].plan.NI, a[l].plan.NJ, false));
   }
   if constexpr (LEVEL == LFM_COMPLEX)
-    return launch<LEVEL, true, kThreadsComplex>(w, threads, smem, stream);
+    return launch<LEVEL, true, kThreadsComplex, kWaveLattices, false>(w, threads, smem, stream);
   else
-    return threads <= 384 ? launch<LEVEL, true, 384>(w, threads, smem, stream)
-                          : launch<LEVEL, true, 512>(w, threads, smem, stream);
+    return threads <= 384
+               ? launch<LEVEL, true, 384, kWaveLattices, false>(w, threads, smem, stream)
+               : launch<LEVEL, true, 512, kWaveLattices, false>(w, threads, smem, stream);
 }
 
 }  // namespace
@@ -662,8 +672,8 @@ static const std::vector<ResidentPlan>& resident_plans(int level, int N) {
   plans.resize(kMaxBlocks + 1);
   const bool cx = level == LFM_COMPLEX;
   const int ns = cx ? 3 : 2, V = kCells, np = (ns * V + 2) / 3;
-  const int N4 = (N + 3) / 4 * 4, RS = N4 + 4;
-  const int field = cx ? kFieldFloats<LFM_COMPLEX> : kFieldFloats<LFM_REAL>;
+  const int RS = (N + 3) / 4 * 4 + 4;
+  const int field = cx ? kFieldFloats<LFM_COMPLEX, false> : kFieldFloats<LFM_REAL, false>;
   const int groups = (N + V - 1) / V;
   for (int nbi = 1; nbi <= std::min(N, kMaxBlocks); ++nbi) {
     for (int nbj = 1; nbj <= std::min(N, kMaxBlocks / nbi); ++nbj) {
@@ -671,18 +681,20 @@ static const std::vector<ResidentPlan>& resident_plans(int level, int N) {
       const int lanes = NJ * groups;
       if (lanes > kMaxThreads) continue;
       const int halo = 2 * (NJ + 2) + 2 * NI;
-      if (4 + (2 * NI * NJ + halo) * RS > field) continue;
-      const int smem = 4 * (ns * field + NI * NJ * N4 + 2 * halo + NI * NJ);
-      if (smem > kSmemBytes) continue;
+      const int rows = 4 + (2 * NI * NJ + halo) * RS;
+      if (rows > field || smem_bytes(level, N, NI, NJ, false) > kSmemBytes) continue;
       for (int segs = 1; segs <= std::min(NI, kMaxThreads / lanes); ++segs) {
         const int warps = (segs * lanes + 31) / 32, planes = (NI + segs - 1) / segs;
         if (32 * warps > (cx ? kThreadsComplex : kMaxThreads)) break;
         const double issue = cx ? 480.0 : 330.0;
         const double t = (planes + 0.5) * std::max((warps + 3) / 4 * issue, cx ? 1200.0 : 900.0) +
                          0.7 * halo * groups * np + 2300.0;
+        const bool small =
+            N <= kSmallEdge && rows <= kFieldFloats<LFM_REAL, true> && 32 * warps <= 384;
+        const int smem = smem_bytes(level, N, NI, NJ, small);
         ResidentPlan& best = plans[nbi * nbj];
         if (best.nbi == 0 || t < best.cycles)
-          best = ResidentPlan{nbi, nbj, NI, NJ, V, segs, warps * 32, RS, smem,
+          best = ResidentPlan{nbi, nbj, NI, NJ, V, segs, warps * 32, RS, smem, small,
                               4 + 8LL * nbi * nbj * 2 * (NI + NJ) * np * groups, t};
       }
     }
@@ -781,8 +793,11 @@ cudaError_t launch_resident_wave(const ResidentArgs* a, int count, cudaStream_t 
 }
 
 cudaError_t launch_resident(const ResidentArgs& a, cudaStream_t stream) {
-  return a.level == LFM_REAL ? launch_level<LFM_REAL>(a, stream)
-                             : launch_level<LFM_COMPLEX>(a, stream);
+  const bool even = a.N % 2 == 0;
+  if (a.level == LFM_REAL)
+    return even ? launch_level<LFM_REAL, true>(a, stream) : launch_level<LFM_REAL, false>(a, stream);
+  return even ? launch_level<LFM_COMPLEX, true>(a, stream)
+              : launch_level<LFM_COMPLEX, false>(a, stream);
 }
 
 }  // namespace lfm

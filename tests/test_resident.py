@@ -287,3 +287,34 @@ def test_warm_graphs_captures_what_evolve_replays(be):
         B.evolve(1)
         B.warm_graphs()
         assert len(B._graphs) == (0 if tuning is None else 4)
+
+
+@pytest.mark.parametrize("level", [REAL, COMPLEX])
+def test_blocks_of_small_lattices_share_an_sm(level):
+    """Shared memory by what a small lattice needs, so that runs on several streams find
+    room beside one another (REAL takes 144 registers a thread, COMPLEX 160)."""
+    for N in range(8, 37):
+        p = plan(level, N)
+        assert 2 * (p["smem"] + 1024) <= 227 * 1024
+        assert 2 * p["threads"] * (160 if level else 144) <= 65536
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("level", [REAL, COMPLEX])
+def test_many_small_lattices_on_many_streams(be, level):
+    import torch
+
+    sizes = [8, 15, 24, 32, 33, 36, 37, 48, 16, 32, 36, 20]
+    pairs = [(_evolver(level, n, n, be), _evolver(level, n, n, be)) for n in sizes]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(be.device) for _ in pairs]
+    for _ in range(3):
+        for (a, _), s in zip(pairs, streams):
+            with torch.cuda.stream(s):
+                a.evolve(200)
+    torch.cuda.synchronize()
+    for a, b in pairs:
+        b.use_graphs = False
+        b.evolve(600)
+        _same(a, b)
+        a.synchronize()
