@@ -63,6 +63,12 @@ struct Packet {
   uint32_t t;
 };
 
+// A packet is read and written as one: .b128 is a scalar type to PTX (sm_70 on), and its
+// memory model takes a strong operation on a scalar as one operation on all the bytes
+// (one on a vector, as ld.v4.b32, as an operation for each element, in any order).  The
+// 16-byte atomic loads and stores of CUDA C++ (__nv_atomic_load, __nv_atomic_store) rest on
+// the same access; written with them the kernel took 6 % less (REAL 33^3) to 4 % more time
+// (COMPLEX 36^3), 1 % more at REAL 32^3.
 __device__ __forceinline__ void st_packet(ulonglong2* p, const Packet& x) {
   unsigned long long lo, hi;
   memcpy(&lo, &x.v[0], 8);
@@ -90,9 +96,11 @@ __device__ __forceinline__ Packet ld_packet(const ulonglong2* p) {
 }
 
 // Whether a packet of VALUES values carries time level t.  Its spare places carry
-// the level as well and are looked at too, so that every word of the load is used:
-// with spare words left unused (REAL, two cells a thread) torn packets were seen,
-// the compiler being free to load less.
+// the level as well and are looked at too, so that every word of the load is used: with
+// spare words left unused (REAL, two cells a thread) packets were seen whose words did
+// not belong together.  The cause was not found; a load made narrower in compilation,
+// where a part of its result is not used, would explain it.  The packets without spare
+// words use all of theirs.
 template <int VALUES>
 __device__ __forceinline__ bool carries(const Packet& x, uint32_t t) {
   bool ok = x.t == t;
