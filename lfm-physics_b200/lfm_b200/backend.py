@@ -19,6 +19,15 @@ from . import _lib
 from .mask import boundary_mask as _host_mask
 
 
+# names of the step calls' arrays in their errors
+_REAL_ARGS = ("psi_in", "psi_prev_in", "chi_in", "chi_prev_in", "boundary_mask",
+              "psi_out", "psi_prev_out", "chi_out", "chi_prev_out")
+_COMPLEX_ARGS = tuple(f"arg{i}" for i in range(13))
+_COLOR_IN = tuple(f"psi_in{i}" for i in range(4))
+_COLOR_CHI_IN = ("chi_in", "chi_prev_in", "boundary_mask")
+_COLOR_OUT = tuple(f"psi_out{i}" for i in range(4))
+_COLOR_CHI_OUT = ("chi_out", "chi_prev_out")
+
 _DEVICE_ARRAY = None
 
 
@@ -130,8 +139,9 @@ class B200Backend:
         _lib.check_device("synchronize", self.device)
 
     # -- argument checks --------------------------------------------------------
-    def _ptrs(self, arrays) -> list[int]:
-        """Checked device pointers of (array, elements, name) triples.
+    def _ptrs(self, arrays, numel: int, names) -> list[int]:
+        """Device pointers of `arrays`, each checked to be `numel` contiguous float32 values
+        on this backend's device.
 
         Every array this backend hands out is a DeviceArray, whose attributes go
         through torch's subclass dispatch: the 65 reads of a COMPLEX step took 100 us
@@ -140,23 +150,22 @@ class B200Backend:
         """
         import torch
 
+        out, device, f32, tensor = [], self.device, torch.float32, torch.Tensor
         with torch._C.DisableTorchFunctionSubclass():
-            return [self._ptr(t, n, what) for t, n, what in arrays]
-
-    def _ptr(self, t, numel: int, what: str) -> int:
-        import torch
-
-        if not isinstance(t, torch.Tensor):
-            raise TypeError(f"{what}: expected a torch CUDA tensor, got {type(t).__name__}")
-        if t.device != self.device:
-            raise ValueError(f"{what}: tensor on {t.device}, backend on {self.device}")
-        if t.dtype != torch.float32:
-            raise TypeError(f"{what}: expected float32, got {t.dtype}")
-        if not t.is_contiguous():
-            raise ValueError(f"{what}: tensor must be contiguous")
-        if t.numel() != numel:
-            raise ValueError(f"{what}: {t.numel()} elements, expected {numel}")
-        return t.data_ptr()
+            for t, what in zip(arrays, names):
+                if not isinstance(t, tensor):
+                    raise TypeError(
+                        f"{what}: expected a torch CUDA tensor, got {type(t).__name__}")
+                if t.device != device:
+                    raise ValueError(f"{what}: tensor on {t.device}, backend on {device}")
+                if t.dtype != f32:
+                    raise TypeError(f"{what}: expected float32, got {t.dtype}")
+                if not t.is_contiguous():
+                    raise ValueError(f"{what}: tensor must be contiguous")
+                if t.numel() != numel:
+                    raise ValueError(f"{what}: {t.numel()} elements, expected {numel}")
+                out.append(t.data_ptr())
+        return out
 
     # -- protocol steps -----------------------------------------------------------
     def step_real(self, psi_in, psi_prev_in, chi_in, chi_prev_in, boundary_mask,
@@ -164,11 +173,9 @@ class B200Backend:
                   N, dt2, kappa, lambda_self, chi0, e0_sq) -> None:
         """One leapfrog step for real E (numpy_backend.py:80-130)."""
         n = N**3
-        names = ("psi_in", "psi_prev_in", "chi_in", "chi_prev_in", "boundary_mask",
-                 "psi_out", "psi_prev_out", "chi_out", "chi_prev_out")
         arrs = (psi_in, psi_prev_in, chi_in, chi_prev_in, boundary_mask,
                 psi_out, psi_prev_out, chi_out, chi_prev_out)
-        ptrs = self._ptrs((a, n, nm) for a, nm in zip(arrs, names))
+        ptrs = self._ptrs(arrs, n, _REAL_ARGS)
         _lib.call("lfm_step_real_f32", *ptrs, int(N), float(dt2), float(kappa),
                   float(lambda_self), float(chi0), float(e0_sq), _stream_handle(self.device))
 
@@ -181,7 +188,7 @@ class B200Backend:
         arrs = (psi_r_in, psi_r_prev_in, psi_i_in, psi_i_prev_in, chi_in, chi_prev_in,
                 boundary_mask, psi_r_out, psi_r_prev_out, psi_i_out, psi_i_prev_out, chi_out,
                 chi_prev_out)
-        ptrs = self._ptrs((a, n, f"arg{i}") for i, a in enumerate(arrs))
+        ptrs = self._ptrs(arrs, n, _COMPLEX_ARGS)
         _lib.call("lfm_step_complex_f32", *ptrs, int(N), float(dt2), float(kappa),
                   float(lambda_self), float(chi0), float(e0_sq), float(epsilon_w),
                   _stream_handle(self.device))
@@ -197,15 +204,15 @@ class B200Backend:
         n = N**3
         psi = (psi_r_in, psi_r_prev_in, psi_i_in, psi_i_prev_in)
         outs = (psi_r_out, psi_r_prev_out, psi_i_out, psi_i_prev_out)
-        p_in = self._ptrs((a, 3 * n, f"psi_in{i}") for i, a in enumerate(psi))
-        p_c = self._ptrs(((chi_in, n, "chi_in"), (chi_prev_in, n, "chi_prev_in"),
-                          (boundary_mask, n, "boundary_mask")))
-        p_out = self._ptrs((a, 3 * n, f"psi_out{i}") for i, a in enumerate(outs))
-        p_co = self._ptrs(((chi_out, n, "chi_out"), (chi_prev_out, n, "chi_prev_out")))
-        sa_in = None if sa_fields_in is None else self._ptrs(
-            ((sa_fields_in, 3 * n, "sa_fields_in"),))[0]
-        sa_out = None if sa_fields_out is None else self._ptrs(
-            ((sa_fields_out, 3 * n, "sa_fields_out"),))[0]
+        p_in = self._ptrs(psi, 3 * n, _COLOR_IN)
+        p_c = self._ptrs((chi_in, chi_prev_in, boundary_mask), n, _COLOR_CHI_IN)
+        p_out = self._ptrs(outs, 3 * n, _COLOR_OUT)
+        p_co = self._ptrs((chi_out, chi_prev_out), n, _COLOR_CHI_OUT)
+        sa_in = sa_out = None
+        if sa_fields_in is not None:
+            sa_in, = self._ptrs((sa_fields_in,), 3 * n, ("sa_fields_in",))
+        if sa_fields_out is not None:
+            sa_out, = self._ptrs((sa_fields_out,), 3 * n, ("sa_fields_out",))
         ctx = self.context.handle if (kappa_tube > 0 and sa_out is not None) else None
         _lib.call("lfm_step_color_f32", ctx, *p_in, *p_c, *p_out, *p_co, int(N), float(dt2),
                   float(kappa), float(lambda_self), float(chi0), float(e0_sq),
