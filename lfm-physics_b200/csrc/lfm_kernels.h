@@ -52,8 +52,8 @@ struct StepArgs {
 
 cudaError_t launch_direct_step(const StepArgs& a, cudaStream_t stream);
 
-// Marching kernels through L1 for lattices of any alignment and N >= 32 (COLOR: 45)
-// (step_march.cu); cudaErrorNotSupported below.
+// Marching kernels through L1 for lattices of any alignment (step_march.cu);
+// cudaErrorNotSupported for the smallest, where the direct kernel is the faster one.
 cudaError_t launch_march_step(const StepArgs& a, cudaStream_t stream);
 
 // Fused 2.5D kernel (N % 4 == 0).  Returns cudaErrorNotSupported when the

@@ -384,8 +384,10 @@ __global__ void __launch_bounds__(256, 2)
   }
 }
 
+int color_tiles(int N) { return (N * ((N + 1) / V) + 255) / 256; }
+
 cudaError_t launch_color(const StepArgs& a, bool pairs, cudaStream_t stream) {
-  const int tiles = (a.N * ((a.N + 1) / V) + 255) / 256;
+  const int tiles = color_tiles(a.N);
   const int64_t work = (int64_t)tiles * a.N;
   // All CTAs resident at once (2 x 148) while that takes ten planes or fewer (110^3: 68.3
   // us with nine, 78 with four, 74 with one), four planes beyond (150^3: 178 with four,
@@ -421,12 +423,29 @@ cudaError_t launch(const StepArgs& a, bool pairs, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
+// Whether the march beats the direct kernel, whose one-cell threads are done sooner on the
+// smallest lattices.  us a step, march / direct (every edge from 32 to 65 measured):
+//
+// - REAL: from 32^3 (32^3 2.53 / 2.64, 33^3 2.51 / 2.86, 48^3 3.39 / 4.05; 30^3 4.2 / 3.2),
+//   COMPLEX from 32^3 by pairs (34^3 3.42 / 3.76, 46^3 3.92 / 4.87) and, compensated,
+//   without (33^3 3.51 / 3.53, 37^3 3.50 / 4.03).
+// - Without pairs COMPLEX, and REAL compensated and split chi, from 43^3: COMPLEX 33^3
+//   3.96 / 3.32, 41^3 4.51 / 3.94, 43^3 4.51 / 4.74; split REAL 41^3 3.84 / 3.50, 43^3
+//   3.82 / 4.15.
+// - COLOR from 45^3 (9.27 / 10.2; 44^3 9.99 / 9.98) to the edge whose planes no longer find
+//   room at once (50^3 8.38 / 11.4; 51^3 15.1 / 11.7, 53^3 15.3 / 11.9) and from 54^3 (13.4 /
+//   14.1), without pairs 59^3 (15.8 / 16.4; 57^3 15.7 / 15.1), on.
+bool marching_pays(const StepArgs& a, bool pairs) {
+  if (a.level == LFM_COLOR)
+    return !a.slab && a.N >= 45 &&
+           (a.N >= (pairs ? 54 : 59) || color_tiles(a.N) * a.N <= 2 * 148);
+  const bool from_32 = pairs || (a.level == LFM_REAL ? !a.comp && !a.split : a.comp != 0);
+  return a.N >= (from_32 ? 32 : 43);
+}
+
 }  // namespace
 
 cudaError_t launch_march_step(const StepArgs& a, cudaStream_t stream) {
-  // Below 32^3 the direct kernel's one-cell threads are done sooner (REAL 30^3: 3.2
-  // against 4.2 us a step; COMPLEX 15^3 to 30^3 4.2 either way).
-  if (a.N < 32) return cudaErrorNotSupported;
   // two cells a thread where every row starts on 8 bytes
   bool pairs = a.N % 2 == 0;
   const void* ptrs[] = {a.pr, a.pi, a.chi, a.pr_prev, a.pi_prev, a.chi_prev, a.pr_out, a.pi_out,
@@ -434,11 +453,8 @@ cudaError_t launch_march_step(const StepArgs& a, cudaStream_t stream) {
                         a.chi_lo, a.chi_lo_prev, a.chi_lo_out, a.sa, a.sa_clip_out,
                         a.energy_out};
   for (const void* p : ptrs) pairs = pairs && (reinterpret_cast<uintptr_t>(p) & 7u) == 0;
-  if (a.level == LFM_COLOR) {
-    // (33^3: direct 6.7, march 8.6; 40^3 7.5, 8.8; 50^3 13.8, 10.7)
-    if (a.N < 45 || a.slab) return cudaErrorNotSupported;
-    return launch_color(a, pairs, stream);
-  }
+  if (!marching_pays(a, pairs)) return cudaErrorNotSupported;
+  if (a.level == LFM_COLOR) return launch_color(a, pairs, stream);
   if (a.level == LFM_REAL)
     return a.split  ? launch<LFM_REAL, kSplit>(a, pairs, stream)
            : a.comp ? launch<LFM_REAL, kComp>(a, pairs, stream)

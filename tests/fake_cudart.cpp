@@ -17,6 +17,11 @@ int device = 0, free_sms = kSms, launches = 0, refusals = 0, shared = 0,
 bool capturing = false;
 cudaError_t last = cudaSuccess;
 std::map<std::pair<int, const void*>, int> limit;  // raised limits: (device, kernel)
+std::map<const void*, const char*>& names() {
+  static std::map<const void*, const char*> m;  // filled while the library is loaded
+  return m;
+}
+const char* last_kernel = "";
 struct Config {
   dim3 grid, block;
   size_t smem;
@@ -35,6 +40,7 @@ cudaError_t launch(const void* kernel, dim3 grid, size_t smem, bool cooperative)
   if (cooperative && (int)grid.x > free_sms) e = cudaErrorCooperativeLaunchTooLarge;
   ++(e == cudaSuccess ? launches : refusals);
   shared = (int)smem;
+  last_kernel = names()[kernel];
   return ret(e);
 }
 }  // namespace
@@ -44,6 +50,7 @@ int fake_launches() { return launches; }
 int fake_allocations() { return allocations; }
 void fake_capture(int on) { capturing = on; }
 int fake_refusals() { return refusals; }
+const char* fake_last_kernel() { return last_kernel; }
 int fake_dynamic_smem() { return shared; }  // of the last launch
 int fake_last_error() { return last; }
 void fake_free_sms(int n) { free_sms = n; }
@@ -130,8 +137,10 @@ void** __cudaRegisterFatBinary(void*) {
 }
 void __cudaRegisterFatBinaryEnd(void**) {}
 void __cudaUnregisterFatBinary(void**) {}
-void __cudaRegisterFunction(void**, const char*, char*, const char*, int, void*, void*, void*,
-                            void*, int*) {}
+void __cudaRegisterFunction(void**, const char* host, char*, const char* name, int, void*, void*,
+                            void*, void*, int*) {
+  names()[host] = name;
+}
 void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
 
 cufftResult cufftDestroy(cufftHandle) { return CUFFT_SUCCESS; }

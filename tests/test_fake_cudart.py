@@ -38,6 +38,7 @@ def fake(fake_path, monkeypatch):
     lib = ctypes.CDLL(str(fake_path))
     for name, args in _lib._SIGNATURES.items():
         getattr(lib, name).argtypes = args
+    lib.fake_last_kernel.restype = ctypes.c_char_p
     lib.lfm_strerror.restype = lib.lfm_last_error_detail.restype = ctypes.c_char_p
     monkeypatch.setattr(_lib, "_lib", lib)
     lib.fake_reset()
@@ -93,6 +94,14 @@ class Lattice:
             _lib.call("lfm_leapfrog_real_comp_f32", *p[:6], *self.mask, self.N, *STEP, None)
         else:
             _lib.call("lfm_leapfrog_complex_comp_f32", *p, *self.mask, self.N, *STEP, 0.1, None)
+
+    def split_step(self):
+        f = [np.zeros(self.N**3 + 4, np.float32) for _ in range(8)]
+        p = [(b.ctypes.data + 15) & ~15 for b in f]
+        name, n = (("lfm_leapfrog_real_split_f32", 6) if self.level == REAL
+                   else ("lfm_leapfrog_complex_split_f32", 8))
+        _lib.call(name, *p[:n], *self.mask, 0, self.N, *STEP,
+                  *(() if self.level == REAL else (0.1,)), None)
 
     def desc(self):
         d = _lib.LatticeDesc()
@@ -190,3 +199,20 @@ def test_a_tuned_batch_plans_its_waves_when_a_run_comes(fake):
     fake.fake_capture(0)
     assert _lib.run_steps("lfm_batch_run", tuned, 4, 0, 0, None) is True
     assert fake.fake_allocations() - start == 2 * with_waves
+
+
+@pytest.mark.parametrize("level,form,direct,marches", [
+    (REAL, "step", (31,), (32, 33, 41, 48)),
+    (REAL, "comp_step", (31, 33, 41), (32, 34, 43)),
+    (REAL, "split_step", (31, 33, 41), (32, 34, 43)),
+    (COMPLEX, "step", (31, 33, 41), (32, 34, 43)),
+    (COMPLEX, "masked_step", (31, 33, 41), (32, 34, 43)),
+    (COMPLEX, "comp_step", (31,), (32, 33, 41)),
+    (COMPLEX, "split_step", (31, 33, 41), (32, 34, 43)),
+    (COLOR, "step", (33, 44, 51, 52, 53, 55, 57), (45, 48, 50, 54, 56, 59, 61))])
+def test_the_smallest_lattices_take_the_direct_kernel(fake, level, form, direct, marches):
+    for n in direct + marches:
+        getattr(Lattice(level, n), form)()
+        want = b"direct_step_kernel" if n in direct else (
+            b"march_color_kernel" if level == COLOR else b"march_step_kernel")
+        assert want in fake.fake_last_kernel(), (n, fake.fake_last_kernel())
