@@ -18,8 +18,8 @@
 // the integer key 4 dist^2, so the march has no division, no square root and little
 // index arithmetic.  COMPLEX 256^3: 112 us, 3.0 TB/s of the 335 MB read; a pass over
 // single cells with all of these per cell took 1060 us, with the march but one cell a
-// thread 147.  It waits for loads: neither the conversions to float64 (32 % of their
-// pipe) nor float64 arithmetic (16 %) fill up.  The partial rows' sum, with a thread a
+// thread 147.  It waits for loads: neither the conversions to float64 (50 % of their
+// pipe) nor float64 arithmetic (23 %) fill up.  The partial rows' sum, with a thread a
 // quantity, took 51 us; with a warp each and eight loads in flight, 5.
 //
 // Each CTA reduces its cells to one row of partials in the scratch buffer; a

@@ -296,9 +296,10 @@ __global__ void __launch_bounds__(kThreads<LEVEL>, 2)
 // Seven stencil fields do not fit into a register queue, so a plane's three planes of
 // rows are loaded for each field in turn; marching along i, a CTA finds two of the
 // three in L1.  Two cells a thread run packed, as in the fused kernel.  Without S_a, us
-// a step, against the direct kernel: 50^3 13.8 -> 10.7, 110^3 97.9 -> 68.3, 150^3 256 ->
-// 178, 210^3 711 -> 458; against the fused kernel's run-time tile: 72^3 33.3 -> 23.3,
-// 144^3 214 -> 156, 160^3 241 -> 211, 192^3 372 -> 346.
+// a step, against the direct kernel: 50^3 11.4 -> 8.4, 110^3 97.9 -> 68.3, 150^3 256 ->
+// 178, 210^3 711 -> 458; against the fused kernel's run-time tile: 72^3 26.3 -> 19.7,
+// 144^3 164 -> 141, 160^3 210 -> 193, 288^3 1272 -> 1093 (the tile where it has warps
+// enough: run_time_tile_pays in step_tma.cu).
 template <bool PAIR>
 __global__ void __launch_bounds__(256, 2)
     march_color_kernel(const __grid_constant__ StepArgs a, int planes, int tiles) {
